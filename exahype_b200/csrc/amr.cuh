@@ -17,6 +17,15 @@
 // up. Restrictions add into the coarse data with atomicAdd, so any number of
 // descendants can be restricted into one ancestor in one launch (the sum order
 // is not fixed).
+//
+// Bound: HBM (the fine data once; the coarse cells stay in L2), reached to a
+// part only: a block's index loads, source loads, passes and stores are one
+// chain, so the rate follows from how many small blocks an SM holds. Reading
+// the first axis from and writing the last one to global memory halves the
+// shared-memory traffic of the copy-in, three ping-pong passes, copy-out form,
+// takes one buffer instead of two and two barriers instead of five:
+// prolongation, restriction and vertex projection of 9^3 <-> 27^3 cells at
+// N = 5 together 266 -> 197 us.
 #pragma once
 #include "aderdg.cuh"
 
@@ -34,71 +43,115 @@ __constant__ double c_amr_fine[3 * kAmrSq];
 __constant__ double c_amr_restr[3 * kAmrSq];
 __constant__ double c_amr_equi[kAmrSq];
 
-// applies a 1-D operator along axis AX (0 = fastest) of a tensor with NAX
-// axes of length b and NV values per node, one thread per line:
-// out[.., m, ..] = sum_n M[m][n] in[.., n, ..], M given as a pointer and
-// row/column strides (compile-time indices: the coefficients are read
-// with uniform addresses); all threads of the block take part
-template <int b, int NAX, int AX, int NV, int RS, int CS>
-__device__ __forceinline__ void apply_axis(const double* in, double* out, const double* M) {
-  constexpr int total = NV * ipow(b, NAX), stride = NV * ipow(b, AX), lines = total / b;
-  for (int it = threadIdx.x; it < lines; it += blockDim.x) {
-    const int lo = it % stride, hi = it / stride;
-    const int base = hi * stride * b + lo;
+// A block works on one tensor of NAX axes with b nodes each and NV values per
+// node: one thread per line of the axis in turn (in ROUNDS rounds where a
+// block has fewer threads than lines). The lines of an axis are disjoint, so
+// every pass works in place in one shared buffer; the first pass reads its
+// lines from global memory and the last one writes its results there.
+// Consecutive threads take consecutive values of the x rows, so the last
+// axis (of two or three) is written coalesced; the first (x) pass reads each row
+// whole, through L1. In the buffer the x rows (b NV values) have a pitch of
+// NV modulo 16, which makes the x pass, whose threads stand NV values apart
+// per row, free of bank conflicts too (half-warps, 64-bit accesses).
+template <int b, int NAX, int NV>
+struct TensorCfg {
+  static constexpr int LINES = NV * ipow(b, NAX - 1), SIZE = LINES * b;
+  static constexpr int ROUNDS = (LINES + 255) / 256;
+  static constexpr int THREADS = ((LINES + ROUNDS - 1) / ROUNDS + 31) / 32 * 32;
+  static constexpr int ROW = b * NV, ROWS = ipow(b, NAX - 1);
+  static constexpr int PITCH = ROW + ((NV - ROW) % 16 + 16) % 16;
+  static constexpr int BUF = ROWS * PITCH;
+  // blocks per SM the register budget leaves room for
+  static constexpr int BLOCKS = b >= 8 ? 768 / THREADS : 1536 / THREADS < 32 ? 1536 / THREADS : 32;
+  // first element and element stride of line `it` of axis AX, rows `pitch` apart
+  template <int AX>
+  static __device__ __forceinline__ int first(int it, int pitch) {
+    if (AX == 0) return it / NV * pitch + it % NV;
+    return it / ROW * (AX == 1 ? b * pitch : pitch) + it % ROW;
+  }
+  template <int AX>
+  static constexpr __device__ int stride(int pitch) { return AX == 0 ? NV : AX == 1 ? pitch : b * pitch; }
+};
+
+// where a pass takes its lines from and where it puts them
+enum class Place { kBuffer, kGlobal, kGlobalAdd };
+
+// out[.., m, ..] = sum_n M[m][n] in[.., n, ..] along axis AX, M given as a
+// constant-memory pointer and row / column strides (compile-time indices: the
+// coefficients are constant-bank operands). `tid` of `THREADS` threads.
+template <class C, int b, int AX, int RS, int CS, Place FROM, Place TO, bool ROLLED = false>
+__device__ __forceinline__ void apply_axis(const double* src, double* dst, double* buf, const double* M, int tid) {
+  constexpr int ROW = C::ROW;
+#pragma unroll 1
+  for (int r = 0; r < C::ROUNDS; r++) {
+    const int it = tid + r * C::THREADS;
+    if (it >= C::LINES) break;
+    const double* in = FROM == Place::kBuffer ? buf + C::template first<AX>(it, C::PITCH)
+                                              : src + C::template first<AX>(it, ROW);
+    double* out = TO == Place::kBuffer ? buf + C::template first<AX>(it, C::PITCH)
+                                       : dst + C::template first<AX>(it, ROW);
+    constexpr int is = C::template stride<AX>(FROM == Place::kBuffer ? C::PITCH : ROW);
+    constexpr int os = C::template stride<AX>(TO == Place::kBuffer ? C::PITCH : ROW);
     double x[b];
 #pragma unroll
-    for (int n = 0; n < b; n++) x[n] = in[base + n * stride];
-#pragma unroll
+    for (int n = 0; n < b; n++) x[n] = FROM == Place::kBuffer ? in[n * is] : __ldg(in + n * is);
+#pragma unroll(ROLLED ? 1 : b)
     for (int m = 0; m < b; m++) {
       double s = 0.0;
 #pragma unroll
       for (int n = 0; n < b; n++) s = fma(M[m * RS + n * CS], x[n], s);
-      out[base + m * stride] = s;
+      if (TO == Place::kGlobalAdd)
+        atomicAdd(out + m * os, s);
+      else
+        out[m * os] = s;
     }
   }
 }
 
-// the operator of each axis in turn (axis k uses mats[k]), ping-ponging
-// between the two buffers; returns the buffer holding the result
-template <int b, int NAX, int NV, int RS, int CS>
-__device__ __forceinline__ double* apply_axes(double* cur, double* nxt, const double* const* mats) {
-  __syncthreads();
-  apply_axis<b, NAX, 0, NV, RS, CS>(cur, nxt, mats[0]);
-  if (NAX == 1) return nxt;
-  __syncthreads();
-  apply_axis<b, NAX, 1, NV, RS, CS>(nxt, cur, mats[1]);
-  if (NAX == 2) return cur;
-  __syncthreads();
-  apply_axis<b, NAX, 2, NV, RS, CS>(cur, nxt, mats[2]);
-  return nxt;
-}
-
 // one axis of a single-level transfer: the digit picks the third; each case
-// has a compile-time table address, so the coefficients are constant-bank
-// operands (prolongation P[n][m], restriction R[m][n])
-template <int N, int NAX, int AX, int NV, bool R>
-__device__ __forceinline__ void transfer_axis(const double* in, double* out, int digit) {
+// has a compile-time table address, so that the coefficients are constant-bank
+// operands (prolongation P[n][m], restriction R[m][n]). DEEP (a level among
+// several, in a loop): one form for the three thirds, its coefficients loaded
+// where they are used -- the compiler would hold all matrices in registers
+// across that loop.
+template <class C, int N, int AX, bool R, Place FROM, Place TO, bool DEEP>
+__device__ __forceinline__ void transfer_axis(const double* src, double* dst, double* buf, int digit, int tid) {
   constexpr int b = N + 1, base = 3 * amr_off(N), RS = R ? b : 1, CS = R ? 1 : b;
   const double* tab = R ? c_amr_restr : c_amr_fine;
-  if (digit == 0)
-    apply_axis<b, NAX, AX, NV, RS, CS>(in, out, tab + base);
-  else if (digit == 1)
-    apply_axis<b, NAX, AX, NV, RS, CS>(in, out, tab + base + b * b);
-  else
-    apply_axis<b, NAX, AX, NV, RS, CS>(in, out, tab + base + 2 * b * b);
+  if constexpr (DEEP)
+    apply_axis<C, b, AX, RS, CS, FROM, TO, true>(src, dst, buf, tab + base + digit * b * b, tid);
+  else if (digit == 0) {
+    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base, tid);
+  } else if (digit == 1) {
+    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base + b * b, tid);
+  } else {
+    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base + 2 * b * b, tid);
+  }
 }
 
-template <int N, int NAX, int NV, bool R>
-__device__ __forceinline__ double* transfer_level(double* cur, double* nxt, const int* digit) {
-  __syncthreads();
-  transfer_axis<N, NAX, 0, NV, R>(cur, nxt, digit[0]);
-  if (NAX == 1) return nxt;
-  __syncthreads();
-  transfer_axis<N, NAX, 1, NV, R>(nxt, cur, digit[1]);
-  if (NAX == 2) return cur;
-  __syncthreads();
-  transfer_axis<N, NAX, 2, NV, R>(cur, nxt, digit[2]);
-  return nxt;
+// barrier of the threads that share one buffer: the block, or a part of it
+// (whole warps) under a hardware barrier of its own
+template <int ID, int THREADS>
+__device__ __forceinline__ void part_sync() {
+  if constexpr (ID == 0)
+    __syncthreads();
+  else
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+
+// the axes of one level in turn
+template <int N, int NAX, int NV, bool R, Place FROM, Place TO, int ID, bool DEEP = false>
+__device__ __forceinline__ void transfer_level(const double* src, double* dst, double* buf, const int* digit, int tid) {
+  using C = TensorCfg<N + 1, NAX, NV>;
+  transfer_axis<C, N, 0, R, FROM, NAX == 1 ? TO : Place::kBuffer, DEEP>(src, dst, buf, digit[0], tid);
+  if constexpr (NAX > 1) {
+    part_sync<ID, C::THREADS>();
+    transfer_axis<C, N, 1, R, Place::kBuffer, NAX == 2 ? TO : Place::kBuffer, DEEP>(src, dst, buf, digit[1], tid);
+  }
+  if constexpr (NAX > 2) {
+    part_sync<ID, C::THREADS>();
+    transfer_axis<C, N, 2, R, Place::kBuffer, TO, DEEP>(src, dst, buf, digit[2], tid);
+  }
 }
 
 // levelDelta in 1..kMaxLevelDelta and every index digit-string in
@@ -114,25 +167,26 @@ __device__ __forceinline__ bool valid_index(int ld, const int* index, int nax) {
   return true;
 }
 
-// one transfer of `nax`-dimensional nodal data (nv values per node) between
-// levels: restrict == false prolongates src (coarse) into dst (fine),
-// restrict == true restricts src (fine) and adds it to dst (coarse)
-template <int N, int NAX, int NV>
-__device__ void amr_transfer(const double* __restrict__ src, double* __restrict__ dst, int levelDelta,
-                             const int* index, bool restrict_, double* bufA, double* bufB) {
-  constexpr int b = N + 1;
-  constexpr int size = NV * ipow(b, NAX);
-  for (int e = threadIdx.x; e < size; e += blockDim.x) bufA[e] = src[e];
+// one transfer of NAX-dimensional nodal data (NV values per node) between
+// levels: R false prolongates src (coarse) into dst (fine), R true restricts
+// src (fine) and adds it to dst (coarse)
+template <int N, int NAX, int NV, bool R, int ID = 0>
+__device__ __forceinline__ void amr_transfer(const double* __restrict__ src, double* __restrict__ dst, int levelDelta,
+                                             const int* index, double* buf, int tid) {
+  constexpr Place TO = R ? Place::kGlobalAdd : Place::kGlobal;
+  if (levelDelta == 1) {  // (block-uniform) the digits are the index
+    transfer_level<N, NAX, NV, R, Place::kGlobal, TO, ID>(src, dst, buf, index, tid);
+    return;
+  }
   int rest[3] = {index[0], index[1], index[2]};
   int sig = 1;
   for (int l = 1; l < levelDelta; l++) sig *= 3;
-  double* cur = bufA;
-  double* nxt = bufB;
+#pragma unroll 1
   for (int l = 0; l < levelDelta; l++) {
     int digit[3] = {0, 0, 0};
 #pragma unroll
     for (int k = 0; k < NAX; k++) {
-      if (!restrict_) {  // most significant digit first
+      if (!R) {  // most significant digit first
         digit[k] = rest[k] / sig;
         rest[k] = rest[k] % sig;
       } else {  // least significant digit first
@@ -141,81 +195,88 @@ __device__ void amr_transfer(const double* __restrict__ src, double* __restrict_
       }
     }
     sig = sig > 1 ? sig / 3 : 1;
-    double* res = restrict_ ? transfer_level<N, NAX, NV, true>(cur, nxt, digit)
-                            : transfer_level<N, NAX, NV, false>(cur, nxt, digit);
-    nxt = res == cur ? nxt : cur;
-    cur = res;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < size; e += blockDim.x) {
-    if (restrict_)
-      atomicAdd(dst + e, cur[e]);
+    if (l > 0) part_sync<ID, TensorCfg<N + 1, NAX, NV>::THREADS>();
+    if (l == 0)
+      transfer_level<N, NAX, NV, R, Place::kGlobal, Place::kBuffer, ID, true>(src, dst, buf, digit, tid);
+    else if (l + 1 < levelDelta)
+      transfer_level<N, NAX, NV, R, Place::kBuffer, Place::kBuffer, ID, true>(src, dst, buf, digit, tid);
     else
-      dst[e] = cur[e];
+      transfer_level<N, NAX, NV, R, Place::kBuffer, TO, ID, true>(src, dst, buf, digit, tid);
   }
-  __syncthreads();  // the buffers may be reused by the caller
 }
 
-// op 0: prolongation, 1: restriction. item k: fine cell fine[k], coarse cell
+// R false: prolongation, true: restriction. item k: fine cell fine[k], coarse cell
 // coarse[k], levelDelta[k], subcell index idx[3k .. 3k+2]
-template <int DIM, int N, int ND>
-__global__ void __launch_bounds__(256) amr_volume_kernel(double* __restrict__ luh_a, const double* __restrict__ luh_b,
-                                                         int n, const int* __restrict__ fine,
-                                                         const int* __restrict__ coarse,
-                                                         const int* __restrict__ level_delta,
-                                                         const int* __restrict__ idx, int op) {
-  constexpr int P = ipow(N + 1, DIM);
-  __shared__ double bufA[P * ND], bufB[P * ND];
+template <int DIM, int N, int ND, bool R>
+__global__ void __launch_bounds__(TensorCfg<N + 1, DIM, ND>::THREADS, TensorCfg<N + 1, DIM, ND>::BLOCKS)
+    amr_volume_kernel(double* __restrict__ luh_a, const double* __restrict__ luh_b, int n,
+                      const int* __restrict__ fine, const int* __restrict__ coarse,
+                      const int* __restrict__ level_delta, const int* __restrict__ idx) {
+  using C = TensorCfg<N + 1, DIM, ND>;
+  __shared__ double buf[C::BUF];
   const int k = blockIdx.x;
   if (k >= n) return;
   const int ld = level_delta[k];
   const int index[3] = {idx[3 * k], idx[3 * k + 1], DIM == 3 ? idx[3 * k + 2] : 0};
+  const size_t f = (size_t)fine[k] * C::SIZE, c = (size_t)coarse[k] * C::SIZE;
   if (!valid_index(ld, index, DIM)) return;
-  if (op == 0)  // luh_a: fine (written), luh_b: coarse
-    amr_transfer<N, DIM, ND>(luh_b + (size_t)coarse[k] * P * ND, luh_a + (size_t)fine[k] * P * ND, ld, index, false,
-                             bufA, bufB);
-  else  // luh_a: coarse (added to), luh_b: fine
-    amr_transfer<N, DIM, ND>(luh_b + (size_t)fine[k] * P * ND, luh_a + (size_t)coarse[k] * P * ND, ld, index, true,
-                             bufA, bufB);
+  // luh_a: fine (written) and luh_b: coarse, or luh_a: coarse (added to) and luh_b: fine
+  amr_transfer<N, DIM, ND, R>(luh_b + (R ? f : c), luh_a + (R ? c : f), ld, index, buf, threadIdx.x);
 }
 
 // faces: item k moves face slot fine[k] <-> coarse[k] (slot = cell * 2 DIM +
-// face) of the state array (ND per node) and the flux array (NV per node)
+// face) of the state array (ND per node) and the flux array (NV per node),
+// the first warps of the block working on the state, the others on the flux
 template <int DIM, int N, int ND, int NV>
-__global__ void __launch_bounds__(256) amr_face_kernel(double* __restrict__ q_a, double* __restrict__ f_a,
-                                                       const double* __restrict__ q_b, const double* __restrict__ f_b,
-                                                       int n, const int* __restrict__ fine,
-                                                       const int* __restrict__ coarse,
-                                                       const int* __restrict__ level_delta,
-                                                       const int* __restrict__ idx, int op) {
-  constexpr int F = ipow(N + 1, DIM - 1);
-  __shared__ double bufA[F * ND], bufB[F * ND];
+struct FaceCfg {
+  using Q = TensorCfg<N + 1, DIM - 1, ND>;
+  using F = TensorCfg<N + 1, DIM - 1, NV>;
+  static constexpr int THREADS = Q::THREADS + F::THREADS;
+};
+template <int DIM, int N, int ND, int NV, bool R>
+__global__ void __launch_bounds__(FaceCfg<DIM, N, ND, NV>::THREADS)
+    amr_face_kernel(double* __restrict__ q_a, double* __restrict__ f_a, const double* __restrict__ q_b,
+                    const double* __restrict__ f_b, int n, const int* __restrict__ fine,
+                    const int* __restrict__ coarse, const int* __restrict__ level_delta,
+                    const int* __restrict__ idx) {
+  using C = FaceCfg<DIM, N, ND, NV>;
+  __shared__ double bufQ[C::Q::BUF], bufF[C::F::BUF];
   const int k = blockIdx.x;
   if (k >= n) return;
   const int ld = level_delta[k];
   const int index[3] = {idx[2 * k], DIM == 3 ? idx[2 * k + 1] : 0, 0};
+  const size_t fs = fine[k], cs = coarse[k];
   if (!valid_index(ld, index, DIM - 1)) return;
-  const bool r = op != 0;
-  const size_t from = r ? fine[k] : coarse[k], to = r ? coarse[k] : fine[k];
-  amr_transfer<N, DIM - 1, ND>(q_b + from * F * ND, q_a + to * F * ND, ld, index, r, bufA, bufB);
-  amr_transfer<N, DIM - 1, NV>(f_b + from * F * NV, f_a + to * F * NV, ld, index, r, bufA, bufB);
+  const size_t from = R ? fs : cs, to = R ? cs : fs;
+  const int tq = threadIdx.x, tf = tq - C::Q::THREADS;
+  if (tf < 0)
+    amr_transfer<N, DIM - 1, ND, R, 1>(q_b + from * C::Q::SIZE, q_a + to * C::Q::SIZE, ld, index, bufQ, tq);
+  else
+    amr_transfer<N, DIM - 1, NV, R, 2>(f_b + from * C::F::SIZE, f_a + to * C::F::SIZE, ld, index, bufF, tf);
 }
 
 // the solution of every cell at its (N+1)^d equidistant vertices (x fastest),
 // one block per cell
 template <int DIM, int N, int ND>
-__global__ void __launch_bounds__(256) plot_vertex_kernel(const double* __restrict__ luh, double* __restrict__ out,
-                                                          int ncells) {
-  constexpr int b = N + 1, P = ipow(b, DIM);
-  __shared__ double bufA[P * ND], bufB[P * ND];
+__global__ void __launch_bounds__(TensorCfg<N + 1, DIM, ND>::THREADS, TensorCfg<N + 1, DIM, ND>::BLOCKS)
+    plot_vertex_kernel(const double* __restrict__ luh, double* __restrict__ out, int ncells) {
+  constexpr int b = N + 1;
+  using C = TensorCfg<b, DIM, ND>;
+  __shared__ double buf[C::BUF];
   const int c = blockIdx.x;
   if (c >= ncells) return;
-  for (int e = threadIdx.x; e < P * ND; e += blockDim.x) bufA[e] = luh[(size_t)c * P * ND + e];
+  const double* src = luh + (size_t)c * C::SIZE;
+  double* dst = out + (size_t)c * C::SIZE;
   const double* E = c_amr_equi + amr_off(N);  // E[n][i]: out[i] = sum_n E[n][i] in[n]
-  const double* mats[3] = {E, E, E};
-  double* cur = apply_axes<b, DIM, ND, 1, b>(bufA, bufB, mats);
+  apply_axis<C, b, 0, 1, b, Place::kGlobal, Place::kBuffer>(src, dst, buf, E, threadIdx.x);
   __syncthreads();
-  for (int e = threadIdx.x; e < P * ND; e += blockDim.x) out[(size_t)c * P * ND + e] = cur[e];
+  if constexpr (DIM == 2) {
+    apply_axis<C, b, 1, 1, b, Place::kBuffer, Place::kGlobal>(src, dst, buf, E, threadIdx.x);
+  } else {
+    apply_axis<C, b, 1, 1, b, Place::kBuffer, Place::kBuffer>(src, dst, buf, E, threadIdx.x);
+    __syncthreads();
+    apply_axis<C, b, 2, 1, b, Place::kBuffer, Place::kGlobal>(src, dst, buf, E, threadIdx.x);
+  }
 }
 
 }  // namespace exa

@@ -173,20 +173,28 @@ struct AmrLaunch {
   static int volume(double* a, const double* b, int n, const int* fine, const int* coarse, const int* ld,
                     const int* idx, int op, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    amr_volume_kernel<DIM, N, ND><<<n, 128, 0, st>>>(a, b, n, fine, coarse, ld, idx, op);
+    constexpr int T = TensorCfg<N + 1, DIM, ND>::THREADS;
+    if (op == 0)
+      amr_volume_kernel<DIM, N, ND, false><<<n, T, 0, st>>>(a, b, n, fine, coarse, ld, idx);
+    else
+      amr_volume_kernel<DIM, N, ND, true><<<n, T, 0, st>>>(a, b, n, fine, coarse, ld, idx);
     EXA_LAUNCHED();
     return EXA_OK;
   }
   static int face(double* qa, double* fa, const double* qb, const double* fb, int n, const int* fine,
                   const int* coarse, const int* ld, const int* idx, int op, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    amr_face_kernel<DIM, N, ND, NV><<<n, 256, 0, st>>>(qa, fa, qb, fb, n, fine, coarse, ld, idx, op);
+    constexpr int T = FaceCfg<DIM, N, ND, NV>::THREADS;
+    if (op == 0)
+      amr_face_kernel<DIM, N, ND, NV, false><<<n, T, 0, st>>>(qa, fa, qb, fb, n, fine, coarse, ld, idx);
+    else
+      amr_face_kernel<DIM, N, ND, NV, true><<<n, T, 0, st>>>(qa, fa, qb, fb, n, fine, coarse, ld, idx);
     EXA_LAUNCHED();
     return EXA_OK;
   }
   static int plot(const double* luh, double* out, int n, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    plot_vertex_kernel<DIM, N, ND><<<n, 256, 0, st>>>(luh, out, n);
+    plot_vertex_kernel<DIM, N, ND><<<n, TensorCfg<N + 1, DIM, ND>::THREADS, 0, st>>>(luh, out, n);
     EXA_LAUNCHED();
     return EXA_OK;
   }

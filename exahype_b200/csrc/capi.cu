@@ -2238,7 +2238,7 @@ struct exa_lmesh {
   int *s = nullptr, *s_prev = nullptr, *cure = nullptr, *fs = nullptr, *has_lim = nullptr, *flags = nullptr;
   int *listA = nullptr, *listF = nullptr, *listP = nullptr;
   double *minB = nullptr, *maxB = nullptr, *lim = nullptr, *lim_prev = nullptr, *luh_prev = nullptr;
-  double *fv_ic = nullptr, *gscratch = nullptr;
+  double* fv_ic = nullptr;
   int muscl_grid = 1;
   size_t LS = 0, PB = 0;  // doubles per FV patch (ghosts included), subcells per cell
   int (*init)(exa_lmesh*, double) = nullptr;
@@ -2287,7 +2287,23 @@ template <int DIM, int N>
 struct LimLaunch {
   using PDE = EulerPDE;
   using L = LimShape<DIM, N>;
-  using MC = MusclCfg<DIM, N>;
+  using MC = typename std::conditional<DIM == 2, MusclCfg<N>, Muscl3Cfg<N>>::type;
+  // The scratch that the kernel-level update asks for per block in 3D: the
+  // evolved states and edge fluxes of a whole patch. The kernel keeps them on
+  // chip; the size stays the interface's, and a call with less is refused.
+  static constexpr size_t kShare =
+      DIM == 2 ? 0 : (size_t)ipow(L::B + 2, 3) * 6 * L::nV + (size_t)3 * (L::B + 1) * L::B * L::B * L::nV;
+  static const void* muscl_fn() {
+    if constexpr (DIM == 2) return (const void*)lim_muscl_kernel<N, PDE>;
+    else return (const void*)lim_muscl3_kernel<N, PDE>;
+  }
+  static void muscl_launch(int grid, cudaStream_t st, const int* list, const int* count, int n, double* lim,
+                           double* lim_prev, double* luh, Geometry g, const double* dt, const int* gate) {
+    if constexpr (DIM == 2)
+      lim_muscl_kernel<N, PDE><<<grid, MC::THREADS, MC::SMEM, st>>>(list, count, n, lim, lim_prev, luh, g, dt, gate);
+    else
+      lim_muscl3_kernel<N, PDE><<<grid, MC::THREADS, MC::SMEM, st>>>(list, count, n, lim, lim_prev, luh, g, dt, gate);
+  }
   using PC = PostCfg<DIM, N>;
   static constexpr int PROJ_TMP = tensor_tmp<DIM, L::b, L::B>() > tensor_tmp<DIM, L::B, L::b>()
                                       ? tensor_tmp<DIM, L::b, L::B>() : tensor_tmp<DIM, L::B, L::b>();
@@ -2297,8 +2313,7 @@ struct LimLaunch {
   static int attrs() {
     static bool done = false;
     if (done) return EXA_OK;
-    EXA_CUDA(cudaFuncSetAttribute(lim_muscl_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)MC::SMEM));
+    EXA_CUDA(cudaFuncSetAttribute(muscl_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MC::SMEM));
     EXA_CUDA(cudaFuncSetAttribute(lim_post_update_kernel<DIM, N, PDE, typename PC::Group>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC::POST_SMEM));
     EXA_CUDA(cudaFuncSetAttribute(lim_init_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2316,49 +2331,40 @@ struct LimLaunch {
   }
   // MUSCL blocks resident on the device at once (grid-stride over the FV list)
   static int muscl_grid(int ncells, int* grid) {
-    EXA_CUDA(cudaFuncSetAttribute(lim_muscl_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)MC::SMEM));
+    EXA_CUDA(cudaFuncSetAttribute(muscl_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MC::SMEM));
     int dev = 0, sms = 0, per_sm = 0;
     EXA_CUDA(cudaGetDevice(&dev));
     EXA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    EXA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lim_muscl_kernel<DIM, N, PDE>, MC::THREADS,
-                                                           MC::SMEM));
+    EXA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, muscl_fn(), MC::THREADS, MC::SMEM));
     *grid = std::max(1, std::min(ncells, sms * std::max(1, per_sm)));
     return EXA_OK;
   }
-  static size_t scratch_doubles() { return MC::kShared ? 0 : (size_t)MC::SCR; }
-
-  // kernel-level entry points (no mesh): MUSCL-Hancock over a cell list with
-  // caller-provided scratch, and the two projections
+  // kernel-level entry points (no mesh): MUSCL-Hancock over a cell list (one
+  // block per cell: the length is known), and the two projections
   static int muscl_call(double* lim, double* lim_old, double* luh, const double* dt, Geometry g, int n,
-                        const int* list, double* scratch, size_t scratch_doubles_avail, cudaStream_t st) {
+                        const int* list, const double* scratch, size_t scratch_doubles_avail, bool needs_scratch,
+                        cudaStream_t st) {
     if (n <= 0) return EXA_OK;
     int rc = attrs();
     if (rc) return rc;
-    int grid = 0;
-    if ((rc = muscl_grid(n, &grid))) return rc;
-    if (!MC::kShared) {
-      const size_t fit = scratch_doubles_avail / (size_t)MC::SCR;
-      if (fit < 1 || !scratch)
+    if constexpr (kShare > 0)
+      if (needs_scratch && (!scratch || scratch_doubles_avail < kShare))
         return fail(EXA_ERR_ARG, "exa_fv_musclhancock_update: scratch holds " +
                                      std::to_string(scratch_doubles_avail * 8) + " bytes, one block needs " +
-                                     std::to_string((size_t)MC::SCR * 8));
-      grid = (int)std::min<size_t>((size_t)grid, fit);
-    }
-    lim_muscl_kernel<DIM, N, PDE><<<grid, MC::THREADS, MC::SMEM, st>>>(list, nullptr, n, lim, lim_old, luh, g, dt,
-                                                                       scratch, nullptr);
+                                     std::to_string(kShare * 8));
+    muscl_launch(n, st, list, nullptr, n, lim, lim_old, luh, g, dt, nullptr);
     EXA_LAUNCHED();
     return EXA_OK;
   }
   static int scratch_bytes_for(int n, size_t* bytes) {
-    if (MC::kShared || n <= 0) {
+    if (kShare == 0 || n <= 0) {
       *bytes = 0;
       return EXA_OK;
     }
     int grid = 0;
     int rc = muscl_grid(n, &grid);
     if (rc) return rc;
-    *bytes = (size_t)grid * MC::SCR * sizeof(double);
+    *bytes = (size_t)grid * kShare * sizeof(double);
     return EXA_OK;
   }
   static int project_call(double* luh, double* lim, int n, const int* list, int to_fv, cudaStream_t st) {
@@ -2408,8 +2414,8 @@ struct LimLaunch {
   }
   static int muscl(exa_lmesh* lm, const int* gate) {
     exa_mesh* m = lm->m;
-    lim_muscl_kernel<DIM, N, PDE><<<lm->muscl_grid, MC::THREADS, MC::SMEM, m->stream>>>(
-        lm->listF, lm->flags + 2, 0, lm->lim, lm->lim_prev, m->luh, m->geo, m->scal + 0, lm->gscratch, gate);
+    muscl_launch(lm->muscl_grid, m->stream, lm->listF, lm->flags + 2, 0, lm->lim, lm->lim_prev, m->luh, m->geo,
+                 m->scal + 0, gate);
     EXA_LAUNCHED();
     return EXA_OK;
   }
@@ -2544,9 +2550,9 @@ struct LimOps {
   int (*step)(exa_lmesh*);
   int (*chunk)(exa_lmesh*, int);
   int (*grid)(int, int*);
-  size_t (*scratch)();
   size_t LS, PB;
-  int (*muscl)(double*, double*, double*, const double*, Geometry, int, const int*, double*, size_t, cudaStream_t);
+  int (*muscl)(double*, double*, double*, const double*, Geometry, int, const int*, const double*, size_t, bool,
+               cudaStream_t);
   int (*scratch_bytes)(int, size_t*);
   int (*project)(double*, double*, int, const int*, int, cudaStream_t);
 };
@@ -2555,7 +2561,7 @@ static bool find_lim_ops(int dim, int order, LimOps* out) {
 #define X(D, NN, PDE_, ID)                                                                              \
   if (dim == D && order == NN) {                                                                        \
     using LL = LimLaunch<D, NN>;                                                                        \
-    *out = LimOps{&LL::init, &LL::step, &LL::chunk, &LL::muscl_grid, &LL::scratch_doubles, (size_t)LimShape<D, NN>::LS, \
+    *out = LimOps{&LL::init, &LL::step, &LL::chunk, &LL::muscl_grid, (size_t)LimShape<D, NN>::LS, \
                   (size_t)LimShape<D, NN>::PB, &LL::muscl_call, &LL::scratch_bytes_for, &LL::project_call};   \
     return true;                                                                                        \
   }
@@ -2611,78 +2617,12 @@ int exa_fv_musclhancock_update(const exa_solver* s, double* lim, double* lim_old
   if (rc) return rc;
   if (!lim || !lim_old || !dt_dev || !dx || ncells < 0)
     return fail(EXA_ERR_ARG, "exa_fv_musclhancock_update: bad argument");
-  return ops.muscl(lim, lim_old, luh, dt_dev, geom(s, dx), ncells, cell_list, (double*)scratch,
-                   scratch_bytes / sizeof(double), (cudaStream_t)stream);
+  return ops.muscl(lim, lim_old, luh, dt_dev, geom(s, dx), ncells, cell_list, (const double*)scratch,
+                   scratch_bytes / sizeof(double), true, (cudaStream_t)stream);
 }
 
-// ---- MUSCL-Hancock without device allocation ---------------------------------
-// exa_fv_musclhancock_update_noalloc runs the same kernel as
-// exa_fv_musclhancock_update with the library's own scratch: a file-scope
-// __device__ array of kNoAllocScratchBytes, found once per device by
-// cudaGetSymbolAddress. The call allocates nothing. Nothing in the array needs
-// to start at zero (every slot a block reads was written by that block for the
-// same cell). Calls that overlap in time share the array and race.
-constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;  // 32 MiB
-static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchBytes / sizeof(double)];
-
-// The current context of the calling thread (the device's primary context
-// once the runtime has touched it), through the driver entry point the
-// runtime exposes, so that the library needs no link against the driver.
-static void* current_context() {
-  typedef int (*CtxGetCurrent)(void**);
-  static CtxGetCurrent fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<CtxGetCurrent>(f);
-  }();
-  void* ctx = nullptr;
-  if (fn && fn(&ctx) != 0) ctx = nullptr;
-  return ctx;
-}
-
-// The device address of g_noalloc_scratch for the current device, looked up
-// with cudaGetSymbolAddress on the first call per device and context (the
-// host-side name of the array is no device address) and cached under the
-// context it was found in: after a reset of the device the module is loaded
-// into a new primary context and the address is looked up again.
-static int noalloc_scratch(double** out) {
-  static std::mutex mu;
-  struct Entry {
-    int dev;
-    void* ctx;
-    double* p;
-  };
-  static std::vector<Entry> per_device;
-  int dev = 0;
-  EXA_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  void* ctx = current_context();
-  for (const auto& e : per_device)
-    if (e.dev == dev && e.ctx == ctx && ctx) {
-      *out = e.p;
-      return EXA_OK;
-    }
-  void* p = nullptr;
-  const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-  if (e != cudaSuccess || !p)
-    return fail(EXA_ERR_CUDA, std::string("exa_fv_musclhancock_update_noalloc: cudaGetSymbolAddress: ") +
-                                  cudaGetErrorString(e));
-  ctx = current_context();  // the lookup makes the runtime's context current if it was not yet
-  for (auto& en : per_device)
-    if (en.dev == dev) {
-      en.ctx = ctx;
-      en.p = static_cast<double*>(p);
-      *out = en.p;
-      return EXA_OK;
-    }
-  per_device.push_back(Entry{dev, ctx, static_cast<double*>(p)});
-  *out = static_cast<double*>(p);
-  return EXA_OK;
-}
-
+// The same kernel without caller scratch: it allocates nothing and keeps its
+// working set on chip.
 int exa_fv_musclhancock_update_noalloc(const exa_solver* s, double* lim, double* lim_old, double* luh,
                                        const double* dt_dev, const double* dx, int ncells, const int* cell_list,
                                        void* stream) {
@@ -2691,15 +2631,8 @@ int exa_fv_musclhancock_update_noalloc(const exa_solver* s, double* lim, double*
   if (rc) return rc;
   if (!lim || !lim_old || !dt_dev || !dx || ncells < 0)
     return fail(EXA_ERR_ARG, "exa_fv_musclhancock_update_noalloc: bad argument");
-  const size_t per_block = ops.scratch() * sizeof(double);
-  if (per_block > kNoAllocScratchBytes)
-    return fail(EXA_ERR_UNSUPPORTED, "exa_fv_musclhancock_update_noalloc: one block of this order needs " +
-                                         std::to_string(per_block) + " bytes of scratch, the static scratch holds " +
-                                         std::to_string(kNoAllocScratchBytes));
-  double* scratch = nullptr;
-  if (per_block > 0 && (rc = noalloc_scratch(&scratch))) return rc;
-  return ops.muscl(lim, lim_old, luh, dt_dev, geom(s, dx), ncells, cell_list, scratch,
-                   kNoAllocScratchBytes / sizeof(double), (cudaStream_t)stream);
+  return ops.muscl(lim, lim_old, luh, dt_dev, geom(s, dx), ncells, cell_list, nullptr, 0, false,
+                   (cudaStream_t)stream);
 }
 
 static void lmesh_free(exa_lmesh* lm) {
@@ -2708,8 +2641,7 @@ static void lmesh_free(exa_lmesh* lm) {
   lm->graph = nullptr;
   for (void* p : {(void*)lm->s, (void*)lm->s_prev, (void*)lm->cure, (void*)lm->fs, (void*)lm->has_lim,
                   (void*)lm->flags, (void*)lm->listA, (void*)lm->listF, (void*)lm->listP, (void*)lm->minB,
-                  (void*)lm->maxB, (void*)lm->lim, (void*)lm->lim_prev, (void*)lm->luh_prev, (void*)lm->fv_ic,
-                  (void*)lm->gscratch})
+                  (void*)lm->maxB, (void*)lm->lim, (void*)lm->lim_prev, (void*)lm->luh_prev, (void*)lm->fv_ic})
     sfree(p, st);
   if (lm->m) exa_mesh_destroy(lm->m);
   lm->m = nullptr;
@@ -2743,15 +2675,13 @@ int exa_lmesh_create(const exa_solver* s, const int* cells, const double* offset
     lmesh_free(lm.get());
     return rc;
   }
-  const size_t scr = ops.scratch();
   cudaStream_t lst = lm->m->stream;
   bool ok = salloc(&lm->s, n * 4, lst) && salloc(&lm->s_prev, n * 4, lst) && salloc(&lm->cure, n * 4, lst) &&
             salloc(&lm->fs, n * D2 * 4, lst) && salloc(&lm->has_lim, n * 4, lst) && salloc(&lm->flags, 8 * 4, lst) &&
             salloc(&lm->listA, n * 4, lst) && salloc(&lm->listF, n * 4, lst) && salloc(&lm->listP, n * 4, lst) &&
             salloc(&lm->minB, n * D2 * 5 * 8, lst) && salloc(&lm->maxB, n * D2 * 5 * 8, lst) &&
             salloc(&lm->lim, n * lm->LS * 8, lst) && salloc(&lm->lim_prev, n * lm->LS * 8, lst) &&
-            salloc(&lm->luh_prev, n * P * 5 * 8, lst) &&
-            (scr == 0 || salloc(&lm->gscratch, (size_t)lm->muscl_grid * scr * 8, lst));
+            salloc(&lm->luh_prev, n * P * 5 * 8, lst);
   if (!ok) {
     cudaGetLastError();
     lmesh_free(lm.get());

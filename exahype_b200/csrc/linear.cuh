@@ -10,23 +10,27 @@
 // The surface integral is the corrector's linear form (aderdg.cuh).
 //
 // The predictor is the Cauchy-Kovalevski procedure: time derivative i+1 of
-// the solution is -sum_d B_d(Q_i) grad_d Q_i, evaluated b times; the time
-// averages over [0, dt] weight derivative i by dt^i / (i+1)!. Per derivative
-// level the cell's state sits in shared memory; the gradients are 1-D line
-// contractions with dudx (one thread per (direction, line, variable)), the
-// non-conservative product and both time averages are per node (one thread
-// per node, accumulators in registers). No iteration and no convergence test.
+// the solution is -sum_d B_d(Q_i) grad_d Q_i, evaluated b-1 times; the time
+// averages over [0, dt] weight derivative i by dt^i / (i+1)!. A linear PDE's
+// coefficients depend on the cell's parameters only, so the time-averaged
+// fluxes need no sums of their own: sum_i w_i B_d grad_d Q_i is B_d applied to
+// the gradient of the time-averaged state, one more gradient pass at the end
+// in the place of 2 d nV running sums per node. No iteration and no
+// convergence test.
+//
+// The cell's state and gradients sit in shared memory as planes, one variable
+// or gradient component of all nodes each, so that the per-node phase reads
+// consecutive doubles. The gradients are 1-D line contractions with dudx (one
+// thread per component and line, the components the product reads), the
+// product and the averages are per node in registers.
+//
+// Bound: the shared-memory pipe (63 accesses per node and level; without the
+// running sums three blocks share an SM). 27^3 N=5 elastic: 1.283 -> 0.757 ms.
 #pragma once
 #include "aderdg.cuh"
+#include "line_tables.cuh"
 
 namespace exa {
-
-// Order of the gradient items, from a shared-memory bank model (64-bit
-// accesses, 16 bank pairs per half-warp) of the gradient phase's strided line
-// accesses: for 3D with 6 or 5 nodes per axis consecutive threads take
-// consecutive lines of one component, elsewhere consecutive components of
-// one line. Odd node strides keep the per-node phase conflict-free.
-constexpr bool ck_line_major(int dim, int b) { return dim == 3 ? b >= 5 : (b == 6 || b == 4); }
 
 // the (direction, variable) gradient components the PDE's ncp reads
 template <class PDE, int DIM>
@@ -48,26 +52,35 @@ struct CKCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
   static constexpr int CPB = cells_per_block<S::P>();
   static constexpr int THREADS = CPB * S::P;
-  static constexpr int LINES = S::P / S::b;          // lines per direction
-  static constexpr int QS = S::nD | 1;          // node stride of the state
-  static constexpr int GS = (DIM * S::nV) | 1;  // node stride of the gradients [d][nV]
-  static constexpr bool LMAJ = ck_line_major(DIM, S::b);
-  static constexpr int SQ = S::P * QS, SG = S::P * GS;
-  static constexpr size_t SMEM = sizeof(double) * (size_t)CPB * (SQ + SG);
-  static constexpr int NPAIRS = GradPairs<PDE, DIM>().n;
-  static constexpr int GITEMS = CPB * NPAIRS * LINES;  // gradient line items per block
-  static constexpr int IPT = (GITEMS + THREADS - 1) / THREADS;
-  static_assert(S::P < 1024 && S::nV <= 16 && CPB <= 16, "packed item descriptors");
+  static constexpr int LINES = S::F;                                             // lines per direction
+  static constexpr int NPAIRS = GradPairs<PDE, DIM>().n, NU = NPAIRS / DIM;  // gradient components, per direction
+  // planes: row pitch (4 nodes: 5, or the x lines' threads would meet in four
+  // banks), plane pitch (odd: the variables of one node lie in different banks)
+  static constexpr int YP = S::b == 4 ? 5 : S::b, ZP = S::b * YP;
+  static constexpr int PL = (ZP * (DIM == 3 ? S::b : 1)) | 1;
+  static constexpr int SC = (S::nD + NPAIRS) * PL;  // doubles per cell
+  static constexpr size_t SMEM = sizeof(double) * (size_t)CPB * SC;
+  // gradient items per thread; with NU == b one direction per round
+  static constexpr int ROUNDS = (NPAIRS + S::b - 1) / S::b;
+  static constexpr bool kDirRounds = NU == S::b;
+  // Blocks per SM of the register budget: three where a block is one cell
+  // (27^3 N=5 0.753 ms, with two 0.793, four 0.775); the 250- and 256-thread
+  // blocks of the lower orders spill there (25x21x19 N=4 0.232 ms with two,
+  // 0.263 with three).
+  static constexpr int BLOCKS = CPB == 1 && !PDE::kPointSource ? 3 : 2;  // (the point source's code needs more)
+  static constexpr int NREG = regs_for_blocks<THREADS, BLOCKS>();
+  static_assert(NU * DIM == NPAIRS, "as many components in every direction");
+  static_assert(S::nD + NU >= 2 * S::nV, "the second direction's fluxes lie behind the first's");
+  static __host__ __device__ constexpr int pos(int x, int y, int z) { return z * ZP + y * YP + x; }
+  static __host__ __device__ constexpr int step(int d) { return d == 0 ? 1 : d == 1 ? YP : ZP; }
+  // first node of line L along d (L enumerates the other coordinates in
+  // (z, y, x) order, the face-node order of the reference)
+  static __device__ __forceinline__ int line0(int d, int L) {
+    const int a = L / S::b, c = L % S::b;
+    if (DIM == 2) return d == 0 ? L * YP : L;
+    return d == 0 ? a * ZP + c * YP : d == 1 ? a * ZP + c : a * YP + c;
+  }
 };
-
-// node of line L along direction d at position n; L enumerates the other
-// coordinates in (z, y, x) order (face-node order of the reference)
-template <int DIM, int b>
-__device__ __forceinline__ int line_node(int d, int L, int n) {
-  const int a0 = L / b, a1 = L % b;
-  if (DIM == 2) return d == 0 ? L * b + n : n * b + L;
-  return d == 0 ? (a0 * b + a1) * b + n : d == 1 ? (a0 * b + n) * b + a1 : (n * b + a0) * b + a1;
-}
 
 // Lagrange basis polynomial i of the Gauss-Legendre nodes of order N at xi
 // (the reference's basisFunctions[N][i], kernels/DGBasisFunctions.h:53), as
@@ -153,18 +166,17 @@ __device__ void node_point_source_sum(const Geometry& geo, const double* c, cons
   }
 }
 
-// NREG: register cap per thread, regs_for_blocks<THREADS, blocks per SM>()
-template <int DIM, int N, class PDE, int NREG>
+template <int DIM, int N, class PDE, int NREG = CKCfg<DIM, N, PDE>::NREG>
 __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     ck_predictor_kernel(const double* __restrict__ luh, double* __restrict__ lQhbnd, double* __restrict__ lFhbnd,
                         double* __restrict__ lduh, const double* __restrict__ dt_ptr, Geometry geo, int ncells,
                         const int* __restrict__ cell_list, const int* __restrict__ count,
                         double* __restrict__ lQhi_out, double* __restrict__ lFhi_out) {
   using C = CKCfg<DIM, N, PDE>;
-  constexpr int b = C::b, P = C::P, nV = C::nV, nD = C::nD, LINES = C::LINES, QS = C::QS, GS = C::GS;
-  constexpr int F = C::F;
+  constexpr int b = C::b, P = C::P, nV = C::nV, nD = C::nD, LINES = C::LINES, PL = C::PL, F = C::F, NU = C::NU;
   extern __shared__ double smem[];
   const OrderTables& T = c_tab[N];
+  const LineTables<N>& K = line_tab<N>();
   const int lc = threadIdx.x / P;
   const int p = threadIdx.x - lc * P;
   const int slot = blockIdx.x * C::CPB + lc;
@@ -172,22 +184,20 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
   if ((int)blockIdx.x * C::CPB >= nact) return;  // whole block, before its first barrier
   const bool active = slot < nact;
   const int cell = active ? (cell_list ? cell_list[slot] : slot) : 0;
-  double* sQ = smem + lc * C::SQ;
-  double* sG = smem + C::CPB * C::SQ + lc * C::SG;
+  double* sC = smem + lc * C::SC;
+  const int x = p % b, y = (p / b) % b, z = DIM == 3 ? p / (b * b) : 0;
+  double* own = sC + C::pos(x, y, z);
+  double* ownG = own + nD * PL;
   const int inst = cell_instance(geo, cell);
   const double dt = dt_ptr[inst];
-  __shared__ double s_idx[C::CPB][3];
-  __shared__ int s_cell[C::CPB];
-  if (p == 0) {
-    s_cell[lc] = active ? cell : -1;
+  double idx[DIM];
 #pragma unroll
-    for (int d = 0; d < 3; d++) s_idx[lc][d] = d < DIM ? 1.0 / cell_width(geo, inst, d) : 0.0;
-  }
+  for (int d = 0; d < DIM; d++) idx[d] = 1.0 / cell_width(geo, inst, d);
   // point sources: this cell's centre, widths and time stamp, and whether
   // the source lies in it (the same for all threads of the cell)
   constexpr bool PS = PDE::kPointSource;
   double pc[3] = {0.0, 0.0, 0.0}, ph[3] = {1.0, 1.0, 1.0}, pt = 0.0;
-  bool src = false;
+  bool here = false;
   if constexpr (PS) {
     if (active && geo.centre) {
 #pragma unroll
@@ -196,199 +206,199 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
         ph[d] = cell_width(geo, inst, d);
       }
       pt = *geo.time;
-      src = point_source_in_cell<DIM, PDE>(geo, pc, ph);
+      here = point_source_in_cell<DIM, PDE>(geo, pc, ph);
     }
   }
-  // level 0: the solution (parameters included); inactive slots get unit
-  // parameters so that their arithmetic stays finite. A point source adds dt
-  // times its time integral (3d/spaceTimePredictorLinear.cpph:77-90).
-  double qh[nV];
+  // level 0: the solution (parameters included), read by consecutive threads;
+  // inactive slots get unit parameters so that their arithmetic stays finite
   {
-    double psw[nV];
+    const double* src = luh + (size_t)cell * P * nD;
 #pragma unroll
-    for (int v = 0; v < nV; v++) psw[v] = 0.0;
-    if constexpr (PS)
-      if (src) node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
-#pragma unroll
-    for (int v = 0; v < nD; v++) {
-      double q = active ? __ldg(luh + ((size_t)cell * P + p) * nD + v) : (v < nV ? 0.0 : 1.0);
-      if (v < nV && PS && src) q = __dadd_rn(q, __dmul_rn(dt, psw[v]));
-      sQ[p * QS + v] = q;
-      if (v < nV) qh[v] = q;
+    for (int k = 0; k < nD; k++) {
+      const int e = p + k * P, n = e / nD, v = e - n * nD;
+      const int nx = n % b, ny = (n / b) % b, nz = DIM == 3 ? n / (b * b) : 0;
+      sC[v * PL + C::pos(nx, ny, nz)] = active ? __ldg(src + e) : (v < nV ? 0.0 : 1.0);
     }
   }
-  double fh[DIM][nV];
-  double fac_i = 0.0, fac_n = 0.5 * dt;  // weights of levels i and i+1 in the time averages
-  // the block's gradient items, packed once: first node of the line (10
-  // bits), direction (2), variable (4), cell of the block (4); item k of
-  // thread t is s_desc[k][t], -1: none
-  __shared__ int s_desc[C::IPT][C::THREADS];
-  // the (direction, variable) pairs, copied with compile-time indices (a
-  // runtime index into the constexpr table would build a copy of it in every
-  // thread's local memory)
-  __shared__ int s_pair[C::NPAIRS];
-  if (threadIdx.x == 0) {
-    constexpr GradPairs<PDE, DIM> GP;
+  // gradient items of this thread: component j of the pairs, line L.
+  // Consecutive threads take consecutive lines of one component; along x
+  // (with one direction per round) consecutive components of one line, whose
+  // lines start an even number of doubles apart.
+  int g_src[C::ROUNDS], g_dst[C::ROUNDS];
 #pragma unroll
-    for (int i = 0; i < C::NPAIRS; i++) s_pair[i] = GP.d[i] | GP.v[i] << 4;
-  }
-  __syncthreads();
-  for (int k = 0; k < C::IPT; k++) {
-    const int it = threadIdx.x + k * C::THREADS;
-    int dsc = -1;
-    if (it < C::GITEMS) {
-      const int L = C::LMAJ ? it % LINES : (it / C::NPAIRS) % LINES;
-      const int pr = C::LMAJ ? (it / LINES) % C::NPAIRS : it % C::NPAIRS;
-      const int c = it / (C::NPAIRS * LINES);
-      const int d = s_pair[pr] & 15, v = s_pair[pr] >> 4;
-      dsc = line_node<DIM, b>(d, L, 0) | d << 10 | v << 12 | c << 16;
+  for (int r = 0; r < C::ROUNDS; r++) {
+    int L, j;
+    if (C::kDirRounds && r == 0) {
+      L = p / NU;
+      j = p % NU;
+    } else {
+      L = p % LINES;
+      j = p / LINES + b * r;
     }
-    s_desc[k][threadIdx.x] = dsc;
+    g_src[r] = -1;
+    g_dst[r] = 0;
+    if (j < C::NPAIRS) {
+      constexpr GradPairs<PDE, DIM> GP;
+      int v = 0;
+#pragma unroll
+      for (int i = 0; i < C::NPAIRS; i++)
+        if (i == j) v = GP.v[i];
+      const int d = j / NU, l0 = C::line0(d, L);
+      g_src[r] = v * PL + l0;
+      g_dst[r] = (nD + j) * PL + l0;
+    }
   }
-  for (int i = 0; i < b; i++) {
-    __syncthreads();  // level i complete in sQ; previous per-node phase done with sG
-    // spatial gradients of level i, one line per item, into sG[node][d][v]
-    // (the components ncp reads)
-#pragma unroll 1
-    for (int k = 0; k < C::IPT; k++) {
-      const int dsc = s_desc[k][threadIdx.x];
-      if (dsc < 0) continue;
-      const int node0 = dsc & 1023, d = (dsc >> 10) & 3, v = (dsc >> 12) & 15, c = dsc >> 16;
-      if (s_cell[c] < 0) continue;
-      const int step = d == 0 ? 1 : d == 1 ? b : b * b;  // node stride along the line
-      const double* q = smem + c * C::SQ + node0 * QS + v;
-      double* g = smem + C::CPB * C::SQ + c * C::SG + node0 * GS + d * nV + v;
-      const double idx = s_idx[c][d];
+  auto gradients = [&]() {
+#pragma unroll
+    for (int r = 0; r < C::ROUNDS; r++) {
+      if (g_src[r] < 0) continue;
+      int st;
+      if (C::kDirRounds) st = C::step(r);
+      else {
+        const int d = (g_dst[r] / PL - nD) / NU;
+        st = d == 0 ? C::step(0) : d == 1 ? C::step(1) : C::step(2);
+      }
+      const double* s = sC + g_src[r];
+      double* g = sC + g_dst[r];
       double f[b];
 #pragma unroll
-      for (int n = 0; n < b; n++) f[n] = idx * q[n * step * QS];
-#pragma unroll
-      for (int l = 0; l < b; l++) {
-        double s = 0.0;
-#pragma unroll
-        for (int n = 0; n < b; n++) s = fma(f[n], T.dudx[l * b + n], s);
-        g[l * step * GS] = s;
-      }
+      for (int n = 0; n < b; n++) f[n] = s[n * st];
+      line_contract<b>(f, K.DP, K.DQ, [&](int l, double a) { g[l * st] = a; });
     }
-    __syncthreads();
-    // per node: non-conservative product one direction at a time (few
-    // registers live), time averages, next level
-    {
-      // level 1 starts from the point source's value at t (:93-101)
-      double qn[nV];
+  };
+  auto product = [&](const double* Qp, int d, double* B) {
+    double G[nV];
 #pragma unroll
-      for (int v = 0; v < nV; v++) qn[v] = 0.0;
-      if constexpr (PS)
-        if (src && i == 0) node_point_source<DIM, N, PDE>(geo, pc, ph, p, pt, dt, 0, qn);
+    for (int v = 0; v < nV; v++) G[v] = 0.0;
+    int i = 0;
 #pragma unroll
-      for (int d = 0; d < DIM; d++) {
-        double B[nV];
-        PDE::ncp_dir(sQ + p * QS, d, sG + p * GS + d * nV, B);
+    for (int v = 0; v < nV; v++)
+      if (PDE::ncp_uses(d, v)) G[v] = idx[d] * ownG[(d * NU + i++) * PL];
+    PDE::ncp_dir(Qp, d, G, B);
+  };
+  __syncthreads();
+  double Qp[nD], qh[nV];  // the node's parameters, the time-averaged state
 #pragma unroll
-        for (int v = 0; v < nV; v++) {
-          fh[d][v] = i == 0 ? B[v] : fma(fac_i, B[v], fh[d][v]);
-          qn[v] -= B[v];
-        }
-      }
-      if (i + 1 < b) {
+  for (int v = 0; v < nV; v++) qh[v] = own[v * PL], Qp[v] = 0.0;
 #pragma unroll
-        for (int v = 0; v < nV; v++) {
-          qh[v] = fma(fac_n, qn[v], qh[v]);
-          sQ[p * QS + v] = qn[v];  // own node only; parameters stay
-        }
-      }
-      fac_i = fac_n;
-      fac_n = fac_n * (dt / (i + 3));
-    }
-  }
+  for (int v = nV; v < nD; v++) Qp[v] = own[v * PL];
   if constexpr (PS) {
-    if (src) {  // the time integral of the source, split over the directions (:294-308)
+    // a point source adds dt times its time integral to level 0
+    // (3d/spaceTimePredictorLinear.cpph:77-90)
+    if (here) {
       double psw[nV];
       node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
 #pragma unroll
-      for (int d = 0; d < DIM; d++)
-#pragma unroll
-        for (int v = 0; v < nV; v++) fh[d][v] = __dadd_rn(fh[d][v], __ddiv_rn(psw[v], (double)DIM));
+      for (int v = 0; v < nV; v++) own[v * PL] = qh[v] = __dadd_rn(qh[v], __dmul_rn(dt, psw[v]));
     }
+    __syncthreads();
   }
-  __syncthreads();
-  // stage the time averages for the extrapolation: lQhi in sQ, lFhi in sG
+  double fac = 0.5 * dt;  // weight of level i + 1 in the time averages
+#pragma unroll 1
+  for (int i = 0; i + 1 < b; i++) {
+    if (i > 0) __syncthreads();  // level i complete
+    gradients();
+    __syncthreads();
+    double qn[nV];
 #pragma unroll
-  for (int v = 0; v < nV; v++) sQ[p * QS + v] = qh[v];
+    for (int v = 0; v < nV; v++) qn[v] = 0.0;
+    if constexpr (PS)  // level 1 starts from the point source's value at t (:93-101)
+      if (here && i == 0) node_point_source<DIM, N, PDE>(geo, pc, ph, p, pt, dt, 0, qn);
 #pragma unroll
-  for (int d = 0; d < DIM; d++)
+    for (int d = 0; d < DIM; d++) {
+      double B[nV];
+      product(Qp, d, B);
 #pragma unroll
-    for (int v = 0; v < nV; v++) sG[p * GS + d * nV + v] = fh[d][v];
-  if (active) {
-    if (lQhi_out)
-      for (int v = 0; v < nD; v++) lQhi_out[((size_t)cell * P + p) * nD + v] = sQ[p * QS + v];
-    if (lFhi_out)  // from the staged copy: indexing fh here would put it in local memory
-      for (int d = 0; d < DIM; d++)
-        for (int v = 0; v < nV; v++) lFhi_out[(((size_t)cell * DIM + d) * P + p) * nV + v] = sG[p * GS + d * nV + v];
-  }
-  __syncthreads();
-  // boundary extrapolation: states (parameters included) and normal fluxes
-  constexpr int QITEMS = C::CPB * DIM * LINES * nD;
-  for (int it = threadIdx.x; it < QITEMS; it += C::THREADS) {
-    const int v = it % nD;
-    const int L = (it / nD) % LINES;
-    const int d = (it / (nD * LINES)) % DIM;
-    const int c = it / (nD * LINES * DIM);
-    const int cc = s_cell[c];
-    if (cc < 0) continue;
-    const double* q = smem + c * C::SQ;
-    double sl = 0.0, sr = 0.0;
-#pragma unroll
-    for (int l = 0; l < b; l++) {
-      const double x = q[line_node<DIM, b>(d, L, l) * QS + v];
-      sl += x * T.FL[l];
-      sr += x * T.FR[l];
+      for (int v = 0; v < nV; v++) qn[v] -= B[v];
     }
-    lQhbnd[(((size_t)cc * 2 * DIM + 2 * d) * F + L) * nD + v] = sl;
-    lQhbnd[(((size_t)cc * 2 * DIM + 2 * d + 1) * F + L) * nD + v] = sr;
-  }
-  constexpr int FITEMS = C::CPB * DIM * LINES * nV;
-  for (int it = threadIdx.x; it < FITEMS; it += C::THREADS) {
-    const int v = it % nV;
-    const int L = (it / nV) % LINES;
-    const int d = (it / (nV * LINES)) % DIM;
-    const int c = it / (nV * LINES * DIM);
-    const int cc = s_cell[c];
-    if (cc < 0) continue;
-    const double* g = smem + C::CPB * C::SQ + c * C::SG;
-    double sl = 0.0, sr = 0.0;
-#pragma unroll
-    for (int l = 0; l < b; l++) {
-      const double x = g[line_node<DIM, b>(d, L, l) * GS + d * nV + v];
-      sl += x * T.FL[l];
-      sr += x * T.FR[l];
-    }
-    lFhbnd[(((size_t)cc * 2 * DIM + 2 * d) * F + L) * nV + v] = sl;
-    lFhbnd[(((size_t)cc * 2 * DIM + 2 * d + 1) * F + L) * nV + v] = sr;
-  }
-  if (!lduh) return;
-  // volumeIntegralLinear from the staged lFhi, staged in turn in the cell's
-  // state buffer and written by consecutive threads to consecutive addresses
-  // (a thread's own nV values would leave every store instruction a partial
-  // write of 32 sectors)
-  __syncthreads();
-  if (active) {
-    const int x = p % b, y = (p / b) % b, z = DIM == 3 ? p / (b * b) : 0;
-    const double w = (DIM == 3 ? T.w[z] * T.w[y] : T.w[y]) * T.w[x];
+    const bool last = i + 2 == b;  // then the averages take the level's place
 #pragma unroll
     for (int v = 0; v < nV; v++) {
-      double du = 0.0;
-#pragma unroll
-      for (int d = 0; d < DIM; d++) du -= w * sG[p * GS + d * nV + v];
-      sQ[p * nV + v] = du;
+      qh[v] = fma(fac, qn[v], qh[v]);
+      own[v * PL] = last ? qh[v] : qn[v];
     }
+    fac = fac * (dt / (i + 3));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < C::CPB * P * nV; i += C::THREADS) {
-    const int c = i / (P * nV), e = i - c * (P * nV);
-    const int cc = s_cell[c];
-    if (cc >= 0) lduh[(size_t)cc * P * nV + e] = smem[c * C::SQ + e];
+  gradients();  // of the time-averaged state, for the fluxes
+  if (lQhi_out && active)
+#pragma unroll
+    for (int v = 0; v < nD; v++) lQhi_out[((size_t)cell * P + p) * nD + v] = v < nV ? qh[v < nV ? v : 0] : Qp[v];
+  // extrapolated states (parameters included), written by consecutive threads
+  double* Qb = lQhbnd + (size_t)cell * 2 * DIM * F * nD;
+  double* Fb = lFhbnd + (size_t)cell * 2 * DIM * F * nV;
+  if (active) {
+#pragma unroll
+    for (int d = 0; d < DIM; d++)
+      for (int it = p; it < LINES * nD; it += P) {
+        const int L = it / nD, v = it - L * nD;
+        const double* q = sC + v * PL + C::line0(d, L);
+        double sl = 0.0, sr = 0.0;
+#pragma unroll
+        for (int l = 0; l < b; l++) {
+          const double a = q[l * C::step(d)];
+          sl += a * T.FL[l];
+          sr += a * T.FR[l];
+        }
+        Qb[2 * d * F * nD + it] = sl;
+        Qb[(2 * d + 1) * F * nD + it] = sr;
+      }
   }
+  __syncthreads();
+  // time-averaged fluxes one direction at a time: the node's values to shared
+  // memory (where nothing is read any more: the state planes, then the planes
+  // behind the first direction's fluxes, then the first's again), their
+  // extrapolation from there; volumeIntegralLinear is pointwise
+  double du[nV];
+  double psw[nV];
+  if constexpr (PS)
+    if (here) node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
+#pragma unroll
+  for (int v = 0; v < nV; v++) du[v] = 0.0;
+  const double w = (DIM == 3 ? T.w[z] * T.w[y] : T.w[y]) * T.w[x];
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    double B[nV];
+    product(Qp, d, B);
+    if constexpr (PS) {  // the time integral of the source, split over the directions (:294-308)
+      if (here)
+#pragma unroll
+        for (int v = 0; v < nV; v++) B[v] = __dadd_rn(B[v], __ddiv_rn(psw[v], (double)DIM));
+    }
+    double* st = sC + (d == 1 ? nV * PL : 0);
+#pragma unroll
+    for (int v = 0; v < nV; v++) {
+      du[v] -= w * B[v];
+      (own + (d == 1 ? nV * PL : 0))[v * PL] = B[v];
+    }
+    if (lFhi_out && active)
+#pragma unroll
+      for (int v = 0; v < nV; v++) lFhi_out[(((size_t)cell * DIM + d) * P + p) * nV + v] = B[v];
+    __syncthreads();
+    if (active)
+      for (int it = p; it < LINES * nV; it += P) {
+        const int L = it / nV, v = it - L * nV;
+        const double* q = st + v * PL + C::line0(d, L);
+        double sl = 0.0, sr = 0.0;
+#pragma unroll
+        for (int l = 0; l < b; l++) {
+          const double a = q[l * C::step(d)];
+          sl += a * T.FL[l];
+          sr += a * T.FR[l];
+        }
+        Fb[2 * d * F * nV + it] = sl;
+        Fb[(2 * d + 1) * F * nV + it] = sr;
+      }
+  }
+  if (!lduh) return;
+  __syncthreads();
+  // staged node by node and written by consecutive threads
+#pragma unroll
+  for (int v = 0; v < nV; v++) sC[p * nV + v] = du[v];
+  __syncthreads();
+  if (active)
+#pragma unroll
+    for (int k = 0; k < nV; k++) lduh[(size_t)cell * P * nV + k * P + p] = sC[k * P + p];
 }
 
 // The linear Riemann solve of one face by one warp: face averages of both

@@ -2226,10 +2226,11 @@ struct exa_lmesh {
   exa_mesh* m = nullptr;  // DG state, faces, stream and time scalars
   int A = 2, T = 3, cure_steps = 0;
   double relax = 1e-4, scale = 1e-3;
-  // s: limiter status; flags: [0] irregular change this step, [1] DG list
-  // length, [2] FV list length, [3] predictor list length, [4] run flag of
-  // run_until's captured step
-  int *s = nullptr, *s_prev = nullptr, *cure = nullptr, *fs = nullptr, *has_lim = nullptr, *flags = nullptr;
+  // s: limiter status, s2: the spreading sweeps' other buffer; flags: [0]
+  // irregular change this step, list lengths: [1] DG, [2] FV, [3] predictor,
+  // [4] FV of the recomputation (0..4 zeroed at the start of a step), [7] run
+  // flag of run_until's captured step
+  int *s = nullptr, *s2 = nullptr, *s_prev = nullptr, *cure = nullptr, *fs = nullptr, *has_lim = nullptr, *flags = nullptr;
   int *listA = nullptr, *listF = nullptr, *listP = nullptr;
   double *minB = nullptr, *maxB = nullptr, *lim = nullptr, *lim_prev = nullptr, *luh_prev = nullptr;
   double* fv_ic = nullptr;
@@ -2238,6 +2239,11 @@ struct exa_lmesh {
   int (*init)(exa_lmesh*, double) = nullptr;
   int (*step)(exa_lmesh*) = nullptr;
   int (*chunk)(exa_lmesh*, int) = nullptr;
+  // Parts of a step that do not depend on one another run beside the mesh
+  // stream: every step forks from it and joins it again, so that the mesh
+  // stream alone orders the steps against everything else.
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t fork = nullptr, ready = nullptr, joined[2] = {nullptr, nullptr};
   cudaGraphExec_t graph = nullptr;  // captured gated step of run_until
   int graph_variant = -1;
   bool initialised = false;
@@ -2371,52 +2377,65 @@ struct LimLaunch {
   }
   static LimParams params(const exa_lmesh* lm) { return LimParams{lm->A, lm->T, lm->cure_steps, lm->relax, lm->scale}; }
 
-  static int select(exa_lmesh* lm, int lo, int hi, int* list, int* count, const int* gate) {
-    exa_mesh* m = lm->m;
-    EXA_CUDA(cudaMemsetAsync(count, 0, sizeof(int), m->stream));
-    lim_select_kernel<<<(m->ncells + 255) / 256, 256, 0, m->stream>>>(m->ncells, lm->s, lo, hi, list, count, gate);
+  // the lists of the cells with lo1 <= s < hi1 and lo2 <= s < hi2 (their
+  // counters are zeroed at the start of the step)
+  static int select2(exa_lmesh* lm, int lo1, int hi1, int* list1, int* count1, int lo2, int hi2, int* list2,
+                     int* count2, const int* gate, cudaStream_t st) {
+    const int n = lm->m->ncells;
+    lim_select2_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, lm->s, lo1, hi1, list1, count1, lo2, hi2, list2, count2, gate);
     EXA_LAUNCHED();
     return EXA_OK;
   }
-  static int merge(exa_lmesh* lm, int minmax, const int* gate) {
+  static constexpr size_t kCounters = 5 * sizeof(int);  // flags[0..4]
+  static int merge(exa_lmesh* lm, const int* gate) {
     exa_mesh* m = lm->m;
     if (m->nfaces <= 0) return EXA_OK;
     lim_merge_faces_kernel<DIM><<<(m->nfaces + 127) / 128, 128, 0, m->stream>>>(
-        m->fl, m->fr, m->fd, m->nfaces, lm->s, lm->minB, lm->maxB, lm->fs, lm->T, minmax, gate);
+        m->fl, m->fr, m->fd, m->nfaces, lm->s, lm->minB, lm->maxB, lm->fs, lm->T, gate);
     EXA_LAUNCHED();
     return EXA_OK;
   }
-  static int spread(exa_lmesh* lm, const int* gate) {  // T sweeps of limiter status spreading
+  // T sweeps of limiter status spreading: T - 2 launches of one sweep, then
+  // one of two sweeps, an even number (T = 2h + 1), which ends in s again
+  static int spread(exa_lmesh* lm, const int* gate) {
     exa_mesh* m = lm->m;
-    for (int it = 0; it < lm->T; it++) {
-      int rc = merge(lm, 0, gate);
-      if (rc) return rc;
-      lim_spread_cells_kernel<DIM, N><<<(m->ncells + 3) / 4, 128, 0, m->stream>>>(
-          m->ncells, lm->s, lm->cure, lm->fs, lm->has_lim, lm->lim, lm->lim_prev, params(lm), gate);
+    CellGrid<DIM> grid;
+    for (int d = 0; d < DIM; d++) {
+      grid.n[d] = m->cells[d];
+      grid.periodic[d] = m->bc[2 * d] == EXA_BC_PERIODIC;
+    }
+    int *from = lm->s, *to = lm->s2;
+    for (int it = 0; it < lm->T - 1; it++) {
+      const int blocks = (m->ncells + 3) / 4;
+      if (it + 2 < lm->T)
+        lim_spread_kernel<DIM, N, 1><<<blocks, 128, 0, m->stream>>>(m->ncells, from, to, lm->cure, lm->has_lim, lm->lim,
+                                                                    lm->lim_prev, grid, params(lm), gate);
+      else
+        lim_spread_kernel<DIM, N, 2><<<blocks, 128, 0, m->stream>>>(m->ncells, from, to, lm->cure, lm->has_lim, lm->lim,
+                                                                    lm->lim_prev, grid, params(lm), gate);
       EXA_LAUNCHED();
+      std::swap(from, to);
     }
     return EXA_OK;
   }
-  static int halo(exa_lmesh* lm, const int* gate) {  // boundary faces: outflow, then reflective (grouped)
+  static int halo(exa_lmesh* lm, const int* gate, cudaStream_t st) {  // boundary faces: outflow, then reflective (grouped)
     exa_mesh* m = lm->m;
     const int nb0 = m->nbfaces[EXA_BC_OUTFLOW], nb = nb0 + m->nbfaces[EXA_BC_REFLECTIVE], total = m->nfaces + nb;
     if (total <= 0) return EXA_OK;
-    lim_fv_halo_kernel<DIM, N><<<(total + 3) / 4, 128, 0, m->stream>>>(
+    lim_fv_halo_kernel<DIM, N><<<(total + 3) / 4, 128, 0, st>>>(
         m->fl, m->fr, m->fd, m->nfaces, m->bcell, m->bface, nb, nb0, lm->s, lm->has_lim, lm->lim, lm->A, gate);
     EXA_LAUNCHED();
     return EXA_OK;
   }
-  static int muscl(exa_lmesh* lm, const int* gate) {
+  static int muscl(exa_lmesh* lm, const int* count, const int* gate, cudaStream_t st) {
     exa_mesh* m = lm->m;
-    muscl_launch(lm->muscl_grid, m->stream, lm->listF, lm->flags + 2, 0, lm->lim, lm->lim_prev, m->luh, m->geo,
+    muscl_launch(lm->muscl_grid, st, lm->listF, count, 0, lm->lim, lm->lim_prev, m->luh, m->geo,
                  m->scal + 0, gate);
     EXA_LAUNCHED();
     return EXA_OK;
   }
-  static int predict(exa_lmesh* lm, const int* run = nullptr) {  // status < T (mappings/Prediction.cpp:176-178)
+  static int predict(exa_lmesh* lm) {  // status < T (mappings/Prediction.cpp:176-178), listed before
     exa_mesh* m = lm->m;
-    int rc = select(lm, INT_MIN, lm->T, lm->listP, lm->flags + 3, run);
-    if (rc) return rc;
     return m->s->k.predictor(m->luh, m->lQhbnd, m->lFhbnd, m->lduh, m->iters, m->scal + 0, m->geo, m->ncells,
                              lm->listP, lm->flags + 3, PredictorTemps{}, false, m->sweeps, m->s->variant, m->stream);
   }
@@ -2429,7 +2448,7 @@ struct LimLaunch {
     lim_scalars_kernel<<<1, 1, 0, m->stream>>>(m->scal, t0);
     EXA_LAUNCHED();
     EXA_CUDA(cudaMemsetAsync(m->sweeps, 0, 8, m->stream));
-    EXA_CUDA(cudaMemsetAsync(lm->flags, 0, 4 * sizeof(int), m->stream));
+    EXA_CUDA(cudaMemsetAsync(lm->flags, 0, kCounters, m->stream));
     lim_init_kernel<DIM, N, PDE><<<n, PC::THREADS, PC::SMEM, m->stream>>>(
         n, m->luh, lm->s, lm->s_prev, lm->cure, lm->fs, lm->has_lim, lm->minB, lm->maxB, params(lm));
     EXA_LAUNCHED();
@@ -2441,6 +2460,9 @@ struct LimLaunch {
       return rc;
     take_dt_kernel<<<1, 1, 0, m->stream>>>(m->scal);
     EXA_LAUNCHED();
+    if ((rc = select2(lm, INT_MIN, lm->T, lm->listP, lm->flags + 3, lm->A, INT_MAX, lm->listF, lm->flags + 4, nullptr,
+                      m->stream)))
+      return rc;
     return predict(lm);
   }
 
@@ -2451,57 +2473,68 @@ struct LimLaunch {
     const KernelSet& k = m->s->k;
     const int n = m->ncells;
     const LimParams prm = params(lm);
-    cudaStream_t st = m->stream;
+    cudaStream_t st = m->stream, dg = lm->side[0], fv = lm->side[1];
     int rc;
-    EXA_CUDA(cudaMemsetAsync(lm->flags, 0, sizeof(int), st));
-    // merge: DMP min/max and facewise statuses; DG Riemann problems (the
-    // fluxes of faces between two FV-active cells are computed but never
-    // read); FV halo exchange and FV boundary on FV-active faces
-    if ((rc = merge(lm, 1, run))) return rc;
-    if ((rc = k.riemann(m->lQhbnd, m->lFhbnd, m->fl, m->fr, m->fd, m->nfaces, run, st))) return rc;
+    EXA_CUDA(cudaMemsetAsync(lm->flags, 0, kCounters, st));
+    EXA_CUDA(cudaEventRecord(lm->fork, st));
+    for (cudaStream_t x : {dg, fv}) EXA_CUDA(cudaStreamWaitEvent(x, lm->fork, 0));
+    // beside one another: the DG Riemann problems (the fluxes of faces between
+    // two FV-active cells are computed but never read), the FV halo exchange
+    // and FV boundary on FV-active faces, and here the copy of the solution
+    // and the lists of DG (s < A) and FV-active cells from the statuses before
+    // the update (the updates do not change them; empty when run holds 0)
+    if ((rc = k.riemann(m->lQhbnd, m->lFhbnd, m->fl, m->fr, m->fd, m->nfaces, run, dg))) return rc;
     for (int kd : {EXA_BC_OUTFLOW, EXA_BC_REFLECTIVE})
       if ((rc = k.boundary(m->lQhbnd, m->lFhbnd, m->bcell + m->boff[kd], m->bface + m->boff[kd], m->nbfaces[kd], kd,
-                           run, st)))
+                           run, dg)))
         return rc;
-    if ((rc = halo(lm, run))) return rc;
-    // update: DG cells (s < A) by the corrector, FV-active cells by
-    // MUSCL-Hancock (lists come out empty when run holds 0)
+    if ((rc = halo(lm, run, fv))) return rc;
+    if ((rc = select2(lm, INT_MIN, lm->A, lm->listA, lm->flags + 1, lm->A, INT_MAX, lm->listF, lm->flags + 2, run, st)))
+      return rc;
     EXA_CUDA(cudaMemcpyAsync(lm->luh_prev, m->luh, (size_t)n * L::P * L::nV * sizeof(double),
                              cudaMemcpyDeviceToDevice, st));
-    // both lists from the statuses before the update (the corrector does not
-    // change them); counters flags[1], flags[2]
-    EXA_CUDA(cudaMemsetAsync(lm->flags + 1, 0, 2 * sizeof(int), st));
-    lim_select2_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, lm->s, INT_MIN, lm->A, lm->listA, lm->flags + 1, lm->A,
-                                                        INT_MAX, lm->listF, lm->flags + 2, run);
-    EXA_LAUNCHED();
+    EXA_CUDA(cudaEventRecord(lm->ready, st));
+    for (cudaStream_t x : {dg, fv}) EXA_CUDA(cudaStreamWaitEvent(x, lm->ready, 0));
+    // update: DG cells by the corrector, FV-active cells by MUSCL-Hancock
+    // (disjoint cells), while the DMP min/max and facewise statuses are merged
     if ((rc = k.corrector(m->luh, m->lduh, m->lFhbnd, m->scal + 0, nullptr, m->geo, n, lm->listA, 1, lm->flags + 1,
-                          st)))
+                          dg)))
       return rc;
-    if ((rc = muscl(lm, run))) return rc;
+    if ((rc = muscl(lm, lm->flags + 2, run, fv))) return rc;
+    if ((rc = merge(lm, run))) return rc;
+    for (int i : {0, 1}) {
+      EXA_CUDA(cudaEventRecord(lm->joined[i], lm->side[i]));
+      EXA_CUDA(cudaStreamWaitEvent(st, lm->joined[i], 0));
+    }
     lim_post_update_kernel<DIM, N, PDE, typename PC::Group>
         <<<(n + PC::CELLS - 1) / PC::CELLS, PC::THREADS, PC::POST_SMEM, st>>>(
         n, m->luh, lm->s, lm->s_prev, lm->cure, lm->fs, lm->has_lim, lm->minB, lm->maxB, lm->lim, lm->lim_prev,
         m->geo, prm, m->scal + 1, lm->flags, run);
     EXA_LAUNCHED();
-    // irregular limiter domain change: every launch below returns at once
-    // unless the post-update kernel raised flags[0] (it never does on a step
-    // that run skips)
+    // irregular limiter domain change: every gated launch below returns at
+    // once unless the post-update kernel raised flags[0] (it never does on a
+    // step that run skips). The lists of the recomputation and of the
+    // predictor need the final statuses only and come beside it.
     const int* g = lm->flags;
     if ((rc = spread(lm, g))) return rc;
+    EXA_CUDA(cudaEventRecord(lm->fork, st));
+    EXA_CUDA(cudaStreamWaitEvent(fv, lm->fork, 0));
+    if ((rc = select2(lm, INT_MIN, lm->T, lm->listP, lm->flags + 3, lm->A, INT_MAX, lm->listF, lm->flags + 4, run, fv)))
+      return rc;
+    EXA_CUDA(cudaEventRecord(lm->joined[1], fv));
     lim_reinit_kernel<DIM, N, typename PC::Group><<<(n + PC::CELLS - 1) / PC::CELLS, 128, PROJ_SMEM * PC::CELLS, st>>>(
-        n, m->luh, lm->luh_prev, lm->s, lm->s_prev, lm->cure,
-                                                          lm->has_lim, lm->lim, lm->lim_prev, prm, g);
+        n, m->luh, lm->luh_prev, lm->s, lm->s_prev, lm->cure, lm->has_lim, lm->lim, lm->lim_prev, prm, g);
     EXA_LAUNCHED();
-    if ((rc = halo(lm, g))) return rc;
-    if ((rc = select(lm, lm->A, INT_MAX, lm->listF, lm->flags + 2, g))) return rc;
-    if ((rc = muscl(lm, g))) return rc;
+    if ((rc = halo(lm, g, st))) return rc;
+    EXA_CUDA(cudaStreamWaitEvent(st, lm->joined[1], 0));
+    if ((rc = muscl(lm, lm->flags + 4, g, st))) return rc;
     lim_recompute_kernel<DIM, N, PDE, typename PC::Group>
         <<<(n + PC::CELLS - 1) / PC::CELLS, 128, PROJ_SMEM * PC::CELLS, st>>>(n, m->luh, lm->luh_prev, lm->s, lm->s_prev,
                                                                   lm->lim, lm->lim_prev, m->geo, prm, m->scal + 4, g);
     EXA_LAUNCHED();
     lim_advance_kernel<<<1, 1, 0, st>>>(m->scal, lm->flags, run);
     EXA_LAUNCHED();
-    return predict(lm, run);
+    return predict(lm);
   }
   static int step(exa_lmesh* lm) { return step_launch(lm, nullptr); }
 
@@ -2518,8 +2551,8 @@ struct LimLaunch {
       lm->graph = nullptr;
       cudaGraph_t g = nullptr;
       EXA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      lim_run_gate_kernel<<<1, 1, 0, st>>>(lm->m->scal, lm->flags + 4);
-      const int rc = step_launch(lm, lm->flags + 4);
+      lim_run_gate_kernel<<<1, 1, 0, st>>>(lm->m->scal, lm->flags + 7);
+      const int rc = step_launch(lm, lm->flags + 7);
       const cudaError_t e = cudaStreamEndCapture(st, &g);
       if (rc || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -2629,11 +2662,33 @@ int exa_fv_musclhancock_update_noalloc(const exa_solver* s, double* lim, double*
                    (cudaStream_t)stream);
 }
 
+// side streams of the mesh stream's priority, and the events that fork and join them
+static cudaError_t lmesh_side_streams(exa_lmesh* lm) {
+  int prio = 0;
+  cudaError_t e = cudaStreamGetPriority(lm->m->stream, &prio);
+  for (cudaStream_t& x : lm->side) {
+    if (x) cudaStreamDestroy(x);
+    x = nullptr;
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio);
+  }
+  for (cudaEvent_t* ev : {&lm->fork, &lm->ready, &lm->joined[0], &lm->joined[1]})
+    if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  return e;
+}
+
 static void lmesh_free(exa_lmesh* lm) {
   cudaStream_t st = lm->m ? lm->m->stream : nullptr;
   if (lm->graph) cudaGraphExecDestroy(lm->graph);
   lm->graph = nullptr;
-  for (void* p : {(void*)lm->s, (void*)lm->s_prev, (void*)lm->cure, (void*)lm->fs, (void*)lm->has_lim,
+  for (cudaStream_t& x : lm->side) {  // (their work is joined to the mesh stream)
+    if (x) cudaStreamDestroy(x);
+    x = nullptr;
+  }
+  for (cudaEvent_t* ev : {&lm->fork, &lm->ready, &lm->joined[0], &lm->joined[1]}) {
+    if (*ev) cudaEventDestroy(*ev);
+    *ev = nullptr;
+  }
+  for (void* p : {(void*)lm->s, (void*)lm->s2, (void*)lm->s_prev, (void*)lm->cure, (void*)lm->fs, (void*)lm->has_lim,
                   (void*)lm->flags, (void*)lm->listA, (void*)lm->listF, (void*)lm->listP, (void*)lm->minB,
                   (void*)lm->maxB, (void*)lm->lim, (void*)lm->lim_prev, (void*)lm->luh_prev, (void*)lm->fv_ic})
     sfree(p, st);
@@ -2670,7 +2725,7 @@ int exa_lmesh_create(const exa_solver* s, const int* cells, const double* offset
     return rc;
   }
   cudaStream_t lst = lm->m->stream;
-  bool ok = salloc(&lm->s, n * 4, lst) && salloc(&lm->s_prev, n * 4, lst) && salloc(&lm->cure, n * 4, lst) &&
+  bool ok = salloc(&lm->s, n * 4, lst) && salloc(&lm->s2, n * 4, lst) && salloc(&lm->s_prev, n * 4, lst) && salloc(&lm->cure, n * 4, lst) &&
             salloc(&lm->fs, n * D2 * 4, lst) && salloc(&lm->has_lim, n * 4, lst) && salloc(&lm->flags, 8 * 4, lst) &&
             salloc(&lm->listA, n * 4, lst) && salloc(&lm->listF, n * 4, lst) && salloc(&lm->listP, n * 4, lst) &&
             salloc(&lm->minB, n * D2 * 5 * 8, lst) && salloc(&lm->maxB, n * D2 * 5 * 8, lst) &&
@@ -2680,6 +2735,12 @@ int exa_lmesh_create(const exa_solver* s, const int* cells, const double* offset
     cudaGetLastError();
     lmesh_free(lm.get());
     return fail(EXA_ERR_NOMEM, "exa_lmesh_create: device allocation failed");
+  }
+  const cudaError_t se = lmesh_side_streams(lm.get());
+  if (se != cudaSuccess) {
+    cudaGetLastError();
+    lmesh_free(lm.get());
+    return fail(EXA_ERR_CUDA, std::string("exa_lmesh_create: ") + cudaGetErrorString(se));
   }
   cudaStream_t st = lm->m->stream;
   EXA_CUDA(cudaMemsetAsync(lm->s, 0, n * 4, st));
@@ -2811,7 +2872,10 @@ int exa_lmesh_set_priority(exa_lmesh* lm, int level) {
     cudaGraphExecDestroy(lm->graph);
     lm->graph = nullptr;
   }
-  return exa_mesh_set_priority(lm->m, level);
+  const int rc = exa_mesh_set_priority(lm->m, level);  // waits for the work queued so far
+  if (rc) return rc;
+  EXA_CUDA(lmesh_side_streams(lm));
+  return EXA_OK;
 }
 
 int exa_lmesh_synchronize(exa_lmesh* lm) {

@@ -291,44 +291,44 @@ struct GroupReduce<WarpGroup> {  // one warp: shuffles
 
 // ---------------------------------------------------------------------------
 // Face merge (mergeSolutionMinMaxOnFace :1654-1690, mergeNeighboursLimiterStatus
-// ADERDGSolver.cpp:2544-2595): one thread per interior face. minmax == 0 only
-// recomputes the facewise statuses (limiter status spreading).
+// ADERDGSolver.cpp:2544-2595): one thread per interior face.
+__host__ __device__ __forceinline__ int merged_face_status(int s1, int s2, int T) {
+  const int a = s1 < T ? s1 : T, b = s2 < T ? s2 : T, m = (a < b ? b : a) - 1;
+  return m > 0 ? m : 0;
+}
 template <int DIM>
 __global__ void lim_merge_faces_kernel(const int* __restrict__ fl, const int* __restrict__ fr,
                                        const int* __restrict__ fd, int nfaces, const int* __restrict__ s,
                                        double* __restrict__ minB, double* __restrict__ maxB, int* __restrict__ fs,
-                                       int T, int minmax, const int* __restrict__ gate) {
+                                       int T, const int* __restrict__ gate) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfaces || (gate && !*gate)) return;
   constexpr int D2 = 2 * DIM;
   const int c1 = fl[f], c2 = fr[f], d = fd[f];
   const int f1 = 2 * d + 1, f2 = 2 * d;
-  const int s1 = s[c1], s2 = s[c2];
-  const int v = max(0, max(min(s1, T), min(s2, T)) - 1);
+  const int v = merged_face_status(s[c1], s[c2], T);
   fs[c1 * D2 + f1] = v;
   fs[c2 * D2 + f2] = v;
-  if (minmax) {
-    double* mn1 = minB + ((size_t)c1 * D2 + f1) * 5;
-    double* mn2 = minB + ((size_t)c2 * D2 + f2) * 5;
-    double* mx1 = maxB + ((size_t)c1 * D2 + f1) * 5;
-    double* mx2 = maxB + ((size_t)c2 * D2 + f2) * 5;
-    // all twenty loads before the first store (the four blocks lie in one
-    // array each, so the compiler could not move a load above a store)
-    double a1[5], a2[5], b1[5], b2[5];
+  double* mn1 = minB + ((size_t)c1 * D2 + f1) * 5;
+  double* mn2 = minB + ((size_t)c2 * D2 + f2) * 5;
+  double* mx1 = maxB + ((size_t)c1 * D2 + f1) * 5;
+  double* mx2 = maxB + ((size_t)c2 * D2 + f2) * 5;
+  // all twenty loads before the first store (the four blocks lie in one
+  // array each, so the compiler could not move a load above a store)
+  double a1[5], a2[5], b1[5], b2[5];
 #pragma unroll
-    for (int i = 0; i < 5; i++) {
-      a1[i] = mn1[i];
-      a2[i] = mn2[i];
-      b1[i] = mx1[i];
-      b2[i] = mx2[i];
-    }
+  for (int i = 0; i < 5; i++) {
+    a1[i] = mn1[i];
+    a2[i] = mn2[i];
+    b1[i] = mx1[i];
+    b2[i] = mx2[i];
+  }
 #pragma unroll
-    for (int i = 0; i < 5; i++) {
-      const double mn = (a2[i] < a1[i]) ? a2[i] : a1[i];
-      const double mx = (b1[i] < b2[i]) ? b2[i] : b1[i];
-      mn1[i] = mn2[i] = mn;
-      mx1[i] = mx2[i] = mx;
-    }
+  for (int i = 0; i < 5; i++) {
+    const double mn = (a2[i] < a1[i]) ? a2[i] : a1[i];
+    const double mx = (b1[i] < b2[i]) ? b2[i] : b1[i];
+    mn1[i] = mn2[i] = mn;
+    mx1[i] = mx2[i] = mx;
   }
 }
 
@@ -571,9 +571,7 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
 //
 // FP64-bound: some 400 operations per subcell of the ring and 250 per edge
 // (slopes, six and two flux evaluations with their divisions, two square
-// roots), 2 M per patch at N = 5. 729 patches with the projection: 847 ->
-// 240 us (with the states and fluxes of the whole patch in 0.7 MB of global
-// scratch per block before, 1 GB of traffic through L2).
+// roots), 2 M per patch at N = 5.
 template <int N>
 struct Muscl3Cfg {
   using L = LimShape<3, N>;
@@ -1124,37 +1122,83 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
   }
 }
 
-// One limiter status spreading sweep, cell part (updateLimiterStatusDuringLimiterStatusSpreading,
-// :392-405); one warp per cell (the status by lane 0, a newly required patch
-// zeroed by the whole warp). The face part is lim_merge_faces_kernel(minmax = 0).
-template <int DIM, int N>
-__global__ void lim_spread_cells_kernel(int ncells, int* __restrict__ s, int* __restrict__ cure,
-                                        int* __restrict__ fs, int* __restrict__ has_lim, double* __restrict__ lim,
-                                        double* __restrict__ lim_prev, LimParams prm, const int* __restrict__ gate) {
+// the uniform mesh's cells, x fastest
+template <int DIM>
+struct CellGrid {
+  int n[DIM];
+  bool periodic[DIM];
+  // the cell across face `face` of cell c, -1: none (a domain boundary)
+  __device__ __forceinline__ int across(int c, int face) const {
+    int at = c, stride = 1;
+    const int d = face >> 1;
+#pragma unroll
+    for (int e = 0; e < DIM; e++)
+      if (e < d) {
+        at /= n[e];
+        stride *= n[e];
+      }
+    int nd = n[0];
+#pragma unroll
+    for (int e = 1; e < DIM; e++) nd = e == d ? n[e] : nd;
+    bool per = periodic[0];
+#pragma unroll
+    for (int e = 1; e < DIM; e++) per = e == d ? periodic[e] : per;
+    const int i = at % nd;
+    if (face & 1) return i + 1 < nd ? c + stride : per ? c - (nd - 1) * stride : -1;
+    return i > 0 ? c - stride : per ? c + (nd - 1) * stride : -1;
+  }
+};
+
+// the status of cell c after one spreading sweep: a cell below T takes the
+// largest merged status of its interior faces
+// (updateLimiterStatusDuringLimiterStatusSpreading, :392-405, after the merge
+// of every face)
+template <int DIM>
+__device__ __forceinline__ int spread_once(const int* __restrict__ s, const CellGrid<DIM>& grid, int c, int T) {
+  const int sc = s[c];
+  if (sc >= T) return T;
+  int ns = 0;
+#pragma unroll
+  for (int f = 0; f < 2 * DIM; f++) {
+    const int o = grid.across(c, f);
+    if (o >= 0) ns = max(ns, merged_face_status(sc, s[o], T));
+  }
+  return ns;
+}
+
+// SWEEPS (1 or 2) limiter status spreading sweeps from s_in to s_out: the
+// merged face statuses of a sweep follow from the statuses on both sides, so
+// a cell's status after two sweeps follows from those of its neighbours'
+// neighbours, without a launch for the faces or between the two. One warp per
+// cell: lanes 0 .. 2 DIM hold the cell and its neighbours; a newly required
+// patch is zeroed by the whole warp.
+template <int DIM, int N, int SWEEPS>
+__global__ void __launch_bounds__(128) lim_spread_kernel(int ncells, const int* __restrict__ s_in,
+                                                         int* __restrict__ s_out, int* __restrict__ cure,
+                                                         int* __restrict__ has_lim, double* __restrict__ lim,
+                                                         double* __restrict__ lim_prev, CellGrid<DIM> grid,
+                                                         LimParams prm, const int* __restrict__ gate) {
   using L = LimShape<DIM, N>;
-  constexpr int D2 = 2 * DIM;
   const int c = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (c >= ncells || (gate && !*gate)) return;
+  // lane f + 1: the cell across face f, after the first sweep
+  const int mine = lane == 0 ? c : lane <= 2 * DIM ? grid.across(c, lane - 1) : -1;
+  int st = -1;
+  if (mine >= 0 && (SWEEPS == 2 || lane == 0)) st = spread_once<DIM>(s_in, grid, mine, prm.T);
+  const int first = __shfl_sync(0xffffffffu, st, 0);
+  int ns = first;
+  if constexpr (SWEEPS == 2) {
+    if (first < prm.T) {
+      ns = lane >= 1 && mine >= 0 ? merged_face_status(first, st, prm.T) : 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ns = max(ns, __shfl_xor_sync(0xffffffffu, ns, o));
+    }
+  }
   int alloc = 0;
   if (lane == 0) {
-    // every load first (one memory round trip), then the status machine
-    const int sc = s[c], hl = has_lim[c];
-    int fsc[D2];
-#pragma unroll
-    for (int i = 0; i < D2; i++) fsc[i] = fs[c * D2 + i];
-    int ns;
-    if (sc < prm.T) {
-      ns = 0;
-#pragma unroll
-      for (int i = 0; i < D2; i++) ns = max(ns, fsc[i]);
-    } else {
-      ns = prm.T;
-      cure[c] = prm.cure_steps + 1;
-    }
-    s[c] = ns;
-#pragma unroll
-    for (int i = 0; i < D2; i++) fs[c * D2 + i] = 0;
-    alloc = ns > 0 && !hl;
+    if (s_in[c] >= prm.T) cure[c] = prm.cure_steps + 1;
+    s_out[c] = ns;
+    alloc = (first > 0 || ns > 0) && !has_lim[c];
     if (alloc) has_lim[c] = 1;
   }
   if (__shfl_sync(0xffffffffu, alloc, 0)) {
@@ -1278,15 +1322,9 @@ __global__ void __launch_bounds__(128) lim_project_kernel(const int* __restrict_
     project_dg_block<DIM, N>(l, u, tmp);
 }
 
-// Compacts the cells whose status satisfies lo <= s < hi into list/count
-// (order is irrelevant: every cell is computed independently).
-__global__ void lim_select_kernel(int ncells, const int* __restrict__ s, int lo, int hi, int* __restrict__ list,
-                                  int* __restrict__ count, const int* __restrict__ gate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gate && !*gate) return;
-  if (c < ncells && s[c] >= lo && s[c] < hi) list[atomicAdd(count, 1)] = c;
-}
-// Two such lists from one pass: lo1 <= s < hi1 and lo2 <= s < hi2.
+// Compacts the cells whose status satisfies lo1 <= s < hi1 into list1/count1
+// and those with lo2 <= s < hi2 into list2/count2 (order is irrelevant: every
+// cell is computed independently).
 __global__ void lim_select2_kernel(int ncells, const int* __restrict__ s, int lo1, int hi1, int* __restrict__ list1,
                                    int* __restrict__ count1, int lo2, int hi2, int* __restrict__ list2,
                                    int* __restrict__ count2, const int* __restrict__ gate) {

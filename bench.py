@@ -61,7 +61,7 @@ def flux_flops(dim):
     return 1 + 5 + 4 + 2 + dim * 9
 
 
-def predictor_flops(dim, N, sweeps, ncells, nV=NVAR, first_sweep_once=False, even_odd=False):
+def predictor_flops(dim, N, sweeps, ncells, nV=NVAR, first_sweep_once=False, even_odd=False, fold_once=False):
     """Algorithmic FLOPs of spaceTimePredictor + volumeIntegral (padding and
     idle lanes not counted): per Picard sweep per cell
     2 d nV b^(d+2) (derivatives) + 2 nV b^(d+2) (iK1) + 2 nV b^(d+1) (rhs0)
@@ -72,13 +72,17 @@ def predictor_flops(dim, N, sweeps, ncells, nV=NVAR, first_sweep_once=False, eve
     starts from the time-constant guess, so its fluxes and derivative
     contractions are formed once instead of once per time slice (1/b). With
     even_odd (b even) each line contraction is the line-form kernel's split
-    into even and odd parts, b^2 + 2 b instead of 2 b^2 flops per line."""
+    into even and odd parts, b^2 + 2 b instead of 2 b^2 flops per line. With
+    fold_once the first sweep's fold through iK1 is two table sums per slice
+    (3 nV b^(d+1) flops) instead of a sum over the slices."""
     b = N + 1
     per_line = b * b + 2 * b if (even_odd and b % 2 == 0) else 2 * b * b
     deriv = dim * nV * b ** dim * per_line + b ** (dim + 1) * flux_flops(dim)
     per_sweep = deriv + 2 * nV * b ** (dim + 2) + 2 * nV * b ** (dim + 1)
     per_cell = 2 * (dim + 2) * nV * b ** (dim + 1) + 8 * dim * nV * b ** dim + 2 * dim * nV * b ** (dim + 1)
     saved = deriv * (b - 1) / b * ncells if first_sweep_once else 0.0
+    if fold_once:
+        saved += (2 * nV * b ** (dim + 2) + 2 * nV * b ** (dim + 1) - 3 * nV * b ** (dim + 1)) * ncells
     return per_sweep * sweeps + per_cell * ncells - saved
 
 
@@ -170,7 +174,8 @@ class ClockSampler:
         return dict(sm_mhz=float(np.median(sm)), sm_max_mhz=mx, reasons=sorted(reasons), samples=len(sm))
 
 
-PREDICTOR_SOURCES = ("exahype_b200/csrc/predictor_lines.cuh", "exahype_b200/csrc/aderdg.cuh",
+PREDICTOR_SOURCES = ("exahype_b200/csrc/predictor_tmem.cuh", "exahype_b200/csrc/line_tables.cuh",
+                     "exahype_b200/csrc/predictor_lines.cuh", "exahype_b200/csrc/aderdg.cuh",
                      "exahype_b200/csrc/pde.cuh", "exahype_b200/csrc/common.cuh", "exahype_b200/csrc/tmem.cuh")
 
 
@@ -390,13 +395,13 @@ def run_ours(a):
     # roofline of the dominant kernel (predictor + volume integral, FP64 pipe)
     ncells = int(np.prod(CELLS))
     pred_ms = ph["predictor"][0] / a.steps
-    line_form = s.variant in (1, 2, 4, 5, 6, 7, 8)  # the line-form kernels form the first sweep once
+    line_form = s.variant != 3  # all but the node form form the first sweep once
     # algorithmic flops: the reference's loops (spaceTimePredictorNonlinear +
     # volumeIntegralNonlinear) for the sweeps the run took; executed: what the
     # chosen kernel does (first sweep once per cell, even/odd contractions)
     pflops = predictor_flops(DIM, ORDER, sweeps / a.steps, ncells)
     pflops_exec = predictor_flops(DIM, ORDER, sweeps / a.steps, ncells, first_sweep_once=line_form,
-                                  even_odd=line_form and s.variant not in (4, 5))
+                                  even_odd=line_form and s.variant not in (4, 5), fold_once=s.variant in (0, 8))
     fp64_peaks = measure_fp64_peak() if not a.no_fp64_probe else None
     fp64_peak = max(fp64_peaks.values()) if fp64_peaks else None
     peaks = load_peaks()

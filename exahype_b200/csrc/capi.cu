@@ -17,6 +17,7 @@
 #include "../../include/exahype_b200.h"
 #include "aderdg.cuh"
 #include "predictor_lines.cuh"
+#include "predictor_tmem.cuh"
 #include "limiter.cuh"
 #include "linear.cuh"
 #include "amr.cuh"
@@ -240,13 +241,16 @@ static int launch_corrector(double* luh, const double* du, const double* fb, con
 }
 
 // Predictor variants the autotuner chooses from (all FP64):
-//   0 node form, 1 block/SM budget    1 line form, 1 block/SM
+//   0 (the default) as variant 8 where that has the shape, else the node form
+//     with the register budget of 1 block/SM
+//   1 line form, 1 block/SM
 //   2 line form, 2 blocks/SM          3 node form, 2 blocks/SM
 //   6 line form, two time slices per phase, 2 blocks/SM
 //   7 line form, two time slices per phase, 1 block/SM
-//   8 line form, Picard iterate in tensor memory, two slices per phase,
-//     2 blocks/SM (orders up to 5 with five state variables; elsewhere as
-//     variant 6)
+//   8 Picard iterate in tensor memory (predictor_tmem.cuh: PDEs of five
+//     state variables without parameters or sources; elsewhere as variant 6).
+//     On every such shape it is faster than the others (its header has the
+//     figures), so it is the default too
 // and the mixed-precision line form (FP32 increment sweeps after the first
 // FP64 sweep), selected explicitly, never by the autotuner:
 //   4 mixed line form, 1 block/SM     5 mixed line form, 2 blocks/SM
@@ -274,18 +278,18 @@ struct Launch {
     return EXA_OK;
   }
 
-  template <bool TEMPS, int MB, bool MIXED = false, int TS = 1, bool TM = false>
+  template <bool TEMPS, int MB, bool MIXED = false, int TS = 1>
   static int launch_lines(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
                           Geometry g, int n, const int* list, const int* cnt, PredictorTemps tmp, cudaStream_t st) {
-    using LC = LinesCfg<DIM, N, PDE, MB, MIXED, TS, TM>;
+    using LC = LinesCfg<DIM, N, PDE, MB, MIXED, TS>;
     static bool attr = false;
     if (!attr) {
-      EXA_CUDA(cudaFuncSetAttribute(predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS, TM>,
+      EXA_CUDA(cudaFuncSetAttribute(predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LC::SMEM));
       attr = true;
     }
     const int grid = (n + LC::CPB - 1) / LC::CPB;
-    predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS, TM>
+    predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS>
         <<<grid, LC::THREADS, LC::SMEM, st>>>(luh, qb, fb, du, iters, dt, g, n, list, tmp, cnt);
     EXA_LAUNCHED();
     return EXA_OK;
@@ -295,23 +299,37 @@ struct Launch {
   static constexpr bool kMixed2 = 2 * LinesCfg<DIM, N, PDE, 2, true>::SMEM <= 227 * 1024;
   static constexpr bool kSlices2 = 2 * LinesCfg<DIM, N, PDE, 2, false, 2>::SMEM <= 227 * 1024;
   static constexpr bool kSlices1 = LinesCfg<DIM, N, PDE, 1, false, 2>::SMEM <= 227 * 1024;
-  // the tensor-memory iterate (variant 8): five doubles per node and slice
-  // (at most 60 columns: N <= 5), a block of whole warps of at most 256 threads
+  // the tensor-memory form (variants 0 and 8)
   using Sh = Shape<DIM, N, PDE>;
-  static constexpr bool kTmemShape = Sh::nD == 5 && Sh::nV == 5 &&
-                                     (cells_per_block<Sh::P>() * Sh::P + 31) / 32 * 32 <= 256 &&
-                                     2 * Sh::b * Sh::nD <= 64;
-  template <int TS>
   static constexpr bool tmem_fits() {
-    if constexpr (kTmemShape) return 2 * LinesCfg<DIM, N, PDE, 2, false, TS, true>::SMEM <= 227 * 1024;
+    if constexpr (Sh::nD == 5 && Sh::nV == 5 && !PDE::kSource && !PDE::kNCP) return TmemCfg<DIM, N, PDE>::kFits;
     else return false;
   }
-  static constexpr bool kTmem2 = tmem_fits<2>();
+  static constexpr bool kTmem = tmem_fits();
+  static int launch_tmem(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
+                         Geometry g, int n, const int* list, const int* cnt, unsigned long long* acc,
+                         cudaStream_t st) {
+    if constexpr (kTmem) {
+      using TC = TmemCfg<DIM, N, PDE>;
+      static bool attr = false;
+      if (!attr) {
+        EXA_CUDA(cudaFuncSetAttribute(predictor_tmem_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)TC::SMEM));
+        attr = true;
+      }
+      predictor_tmem_kernel<DIM, N, PDE><<<(n + TC::CPB - 1) / TC::CPB, TC::THREADS, TC::SMEM, st>>>(
+          luh, qb, fb, du, iters, acc, dt, g, n, list, cnt);
+      EXA_LAUNCHED();
+    }
+    return EXA_OK;
+  }
 
   static int predictor(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
                        Geometry g, int n, const int* list, const int* cnt, PredictorTemps tmp, bool temps,
                        unsigned long long* acc, int variant, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
+    if (kTmem && !temps && (variant == 0 || variant == 8))  // (counts its sweeps itself)
+      return launch_tmem(luh, qb, fb, du, iters, dt, g, n, list, cnt, acc, st);
     int rc;
     if constexpr (PDE::kSource || PDE::kNCP)  // source terms: the node form (1 or 2 blocks per SM)
       rc = temps ? launch_pred<true, 1, 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st)
@@ -330,8 +348,6 @@ struct Launch {
       rc = launch_lines<false, 1, true>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
     else if (variant == 5)
       rc = launch_lines<false, kMixed2 ? 2 : 1, true>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
-    else if (variant == 8 && kTmem2)
-      rc = launch_lines<false, 2, false, 2, kTmem2>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
     else if ((variant == 6 || variant == 8) && kSlices2)
       rc = launch_lines<false, 2, false, kSlices2 ? 2 : 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
     else if (variant == 6 || variant == 7 || variant == 8)

@@ -14,14 +14,21 @@
 
 namespace exa {
 
+// aligned to a line of the constant cache: what one order's kernel reads lies
+// together (unaligned or spread over the constant bank the same operands cost
+// the predictor up to a fifth of its time)
 template <int N>
-struct LineTables {
+struct alignas(256) LineTables {
   static constexpr int b = N + 1, h = b / 2, M = b % 2 == 0 ? h * h : b * b;
+  double KP[M], KQ[M];  // M[n][l] = Kxi[n][l] / w[l]: Picard contraction
+  double VP[M], VQ[M];  // M[m][k] = Kxi[k][m] / w[k]: volume integral
+  double niK1w[b * b];  // [t][l]: -iK1[l][t] w[t]
+  // sum_t iK1[l][t] FL[t] and -sum_t iK1[l][t] w[t]: the first Picard sweep
+  double alpha[b], beta[b];
+  double w[b], FL[b], FR[b];
   double DP[M], DQ[M];  // M[n][l] = dudx[l][n]: derivative at node l
 };
-// The orders the line kernels are instantiated for, in constant memory; what
-// one order's kernel reads lies together (spread over the constant bank the
-// same operands cost the predictor up to a fifth of its time).
+// The orders the line kernels are instantiated for, in constant memory.
 struct LineTablesAll {
   LineTables<3> n3;
   LineTables<4> n4;
@@ -53,7 +60,20 @@ void fill_line_tables(const OrderTables& T, LineTables<N>& L) {
         for (int l = 0; l < b; l++) p[n * b + l] = q[n * b + l] = m(n, l);
     }
   };
+  split([&](int n, int l) { return T.Kxi[n * b + l] / T.w[l]; }, L.KP, L.KQ);
+  split([&](int m, int k) { return T.Kxi[k * b + m] / T.w[k]; }, L.VP, L.VQ);
   split([&](int n, int l) { return T.dudx[l * b + n]; }, L.DP, L.DQ);
+  for (int l = 0; l < b; l++) {
+    L.w[l] = T.w[l];
+    L.FL[l] = T.FL[l];
+    L.FR[l] = T.FR[l];
+    L.alpha[l] = L.beta[l] = 0.0;
+    for (int t = 0; t < b; t++) {
+      L.niK1w[t * b + l] = -T.iK1[l * b + t] * T.w[t];
+      L.alpha[l] += T.iK1[l * b + t] * T.FL[t];
+      L.beta[l] -= T.iK1[l * b + t] * T.w[t];
+    }
+  }
 }
 
 // out(l, sum_n f_n M[n][l]) for every l, M given by its P and Q

@@ -19,22 +19,8 @@
 //   C  one thread per node adds its three directional contributions to the
 //      rhs and folds the rhs into its Picard accumulators through iK1.
 // Shared memory per cell: lQi [P][b][nD], one line-major slice, residuals.
-//
-// TM (five state variables, at most 60 columns per thread): the Picard
-// iterate lQi lives in tensor memory instead (tmem.cuh: each thread owns one
-// TMEM lane, 60 columns of it), so that its reads and writes (phase A, the
-// residual, the update, the time average) leave the shared-memory pipe,
-// which bounds this kernel. The tensor-memory instructions are
-// warp-collective, so the block is rounded up to whole warps (3D N=5, 216
-// nodes: 224 threads; 2D N=5, seven cells of 36: 256); the threads without
-// a node take part in those instructions and in the phase-B items only.
-// With several cells per block a warp can hold nodes of cells in different
-// states (iterating, converged), so there every tensor-memory instruction is
-// issued under block-uniform control only, and per-cell work is selected by
-// the data (a converged cell stores its unchanged iterate back).
 #pragma once
 #include "aderdg.cuh"
-#include "tmem.cuh"
 
 namespace exa {
 
@@ -61,11 +47,11 @@ constexpr bool line_swap_dir(int b, int dim, int nv, int d) { return dim == 3 &&
 // node's last FP32 update in shared memory, SD doubles per cell.
 // TS: time slices per phase (each phase of a Picard sweep handles TS slices
 // between two barriers; TS slice buffers per cell).
-template <int DIM, int N, class PDE, int MINB, bool MIXED = false, int TS = 1, bool TM = false>
+template <int DIM, int N, class PDE, int MINB, bool MIXED = false, int TS = 1>
 struct LinesCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
   static constexpr int CPB = cells_per_block<S::P>();
-  static constexpr int THREADS = TM ? (CPB * S::P + 31) / 32 * 32 : CPB * S::P;
+  static constexpr int THREADS = CPB * S::P;
   static constexpr int LINES = S::P / S::b;  // lines per direction = face nodes
   static constexpr int SR = S::P + 1;
   static constexpr int SD = MIXED ? (S::P * S::b * S::nV + 1) / 2 : 0;
@@ -78,15 +64,7 @@ struct LinesCfg : Shape<DIM, N, PDE> {
   static constexpr bool kPad =
       sizeof(double) * (size_t)(CPB * (S::P * (S::b * S::nD + 1) + TS * SFJ0 + SR + SD)) <= 227 * 1024;
   static constexpr int QS = kPad ? S::b * S::nD + 1 : S::b * S::nD;  // lQi node stride
-  // TM: 32-bit columns per thread and per CTA (the warps of a lane quadrant
-  // take consecutive column ranges)
-  static constexpr int TCOL = 64;
-  static constexpr int TCOLS = TCOL * ((THREADS / 32 + 3) / 4);
-  static_assert(!TM || (!MIXED && S::nD == 5 && S::nV == 5 && 2 * S::b * S::nD <= TCOL && THREADS <= 256),
-                "tensor-memory iterate: five doubles per node and slice, at most 256 threads");
-  // lQi region (TM: none; the region later holds the time-averaged state and
-  // the staged volume integral of every node)
-  static constexpr int SQ = TM ? S::P * (S::nD > S::nV ? S::nD : S::nV) : S::P * QS;
+  static constexpr int SQ = S::P * QS;  // lQi region
   // per direction d: stride along the line, first element, line order
   static constexpr __host__ __device__ int sstride(int d) {
     return kPad ? (d == 0 ? SS0 : d == 1 ? SS1 : SS2) : LINES * S::nV;
@@ -125,15 +103,14 @@ __device__ __forceinline__ int line_swapped(bool swap, int L) { return swap ? (L
 // cancels in the difference, so FP32 only ever carries the increments, whose
 // rounding (relative 6e-8 of the update) is far below the stop test's scale.
 // The stop test and the outputs are as in the FP64 form.
-template <int DIM, int N, class PDE, bool TEMPS, int MINB, bool MIXED = false, int TS = 1, bool TM = false>
-__global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::THREADS, MINB)
+template <int DIM, int N, class PDE, bool TEMPS, int MINB, bool MIXED = false, int TS = 1>
+__global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS>::THREADS, MINB)
     predictor_lines_kernel(const double* __restrict__ luh, double* __restrict__ lQhbnd, double* __restrict__ lFhbnd,
                            double* __restrict__ lduh, int* __restrict__ iters, const double* __restrict__ dt_ptr,
                            Geometry geo, int ncells, const int* __restrict__ cell_list, PredictorTemps tmp,
                            const int* __restrict__ count) {
-  using C = LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>;
+  using C = LinesCfg<DIM, N, PDE, MINB, MIXED, TS>;
   static_assert(!MIXED || TS == 1, "the mixed form works one slice at a time");
-  static_assert(!TM || !TEMPS, "the tensor-memory form writes no temporaries");
   constexpr int b = C::b, P = C::P, nV = C::nV, nD = C::nD, LINES = C::LINES, QS = C::QS;
   extern __shared__ double smem[];
   const OrderTables& T = c_tab[N];
@@ -141,28 +118,13 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
   // a device-side count that leaves this block without cells: the whole
   // block returns before its first barrier (a gated launch costs little)
   if (count && (int)blockIdx.x * C::CPB >= min(*count, ncells)) return;
-  const int lc = TM ? min((int)threadIdx.x / P, C::CPB - 1) : threadIdx.x / P;
+  const int lc = threadIdx.x / P;
   const int p = threadIdx.x - lc * P;
-  const bool nd_ok = !TM || p < P;  // TM: the threads past the last node hold none
-  constexpr bool kTMany = TM && C::CPB > 1;  // tensor memory, several cells per block
-  // TM: the CTA's tensor memory (warp 0 allocates it here and frees it after
-  // the last read of the iterate)
-  const int warp = threadIdx.x >> 5;
-  constexpr bool tm = TM;
-  __shared__ uint32_t s_tbase;
-  uint32_t taddr = 0;
-  if constexpr (TM) {
-    if (warp == 0) tmem::alloc(&s_tbase, C::TCOLS);
-    tmem::fence_before_sync();
-    __syncthreads();
-    tmem::fence_after_sync();
-    taddr = s_tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(C::TCOL * (warp >> 2));
-  }
   const int slot = blockIdx.x * C::CPB + lc;
   const bool active = slot < (count ? min(*count, ncells) : ncells);  // count: optional device-side list length
   const int cell = active ? (cell_list ? cell_list[slot] : slot) : 0;
   double* sQ = smem + lc * C::SQ;
-  double* sQn = sQ + p * QS;  // this node's iterate (not TM)
+  double* sQn = sQ + p * QS;  // this node's iterate
   double* sF = smem + C::CPB * C::SQ + lc * C::SF;
   double* sR = smem + C::CPB * (C::SQ + C::SF) + lc * C::SR;
   double* sFall = smem + C::CPB * C::SQ;
@@ -205,25 +167,12 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
   // slice t of this node's iterate: load (nD values), store (the nV variables
   // the iteration updates; the parameters keep their initial values)
   auto q_ld = [&](int t, double* Q) {
-    if (tm) {
-      uint32_t r[10];
-      tmem::ld10(taddr + 10u * t, r);
-      tmem::wait_ld(r);
-      tmem::unpack5(r, Q);
-    } else {
 #pragma unroll
-      for (int v = 0; v < nD; v++) Q[v] = sQn[t * nD + v];
-    }
+    for (int v = 0; v < nD; v++) Q[v] = sQn[t * nD + v];
   };
   auto q_st = [&](int t, const double* Q) {
-    if (tm) {
-      uint32_t r[10];
-      tmem::pack5(Q, r);
-      tmem::st10(taddr + 10u * t, r);
-    } else {
 #pragma unroll
-      for (int v = 0; v < nV; v++) sQn[t * nD + v] = Q[v];
-    }
+    for (int v = 0; v < nV; v++) sQn[t * nD + v] = Q[v];
   };
 
   double lu[nV];
@@ -231,19 +180,13 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
     const double* src = luh + ((size_t)cell * P + p) * nD;
     double q[nD];
 #pragma unroll
-    for (int v = 0; v < nD; v++) q[v] = active && nd_ok ? __ldg(src + v) : 0.0;
+    for (int v = 0; v < nD; v++) q[v] = active ? __ldg(src + v) : 0.0;
 #pragma unroll
     for (int v = 0; v < nV; v++) lu[v] = q[v];
 #pragma unroll
-    for (int t = 0; t < b; t++) {
-      if (tm) {
-        q_st(t, q);  // nD == nV
-      } else {
+    for (int t = 0; t < b; t++)
 #pragma unroll
-        for (int v = 0; v < nD; v++) sQn[t * nD + v] = q[v];
-      }
-    }
-    if (tm) tmem::wait_st();
+      for (int v = 0; v < nD; v++) sQn[t * nD + v] = q[v];
   }
 
   // Which cells of the block still iterate; phase B skips converged cells.
@@ -306,14 +249,13 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
 #pragma unroll
           for (int v = 0; v < nV; v++)
             sF32[sa[d] + v] = (float)(Fl[d][v] - Fp[d][v]);
-      } else if (kTMany || !done) {
+      } else if (!done) {
 #pragma unroll
         for (int j = 0; j < TS; j++) {
           const int t = t0 + j;
           if (t < b && !(first && j > 0)) {
             double Q[nD];
-            q_ld(t, Q);  // kTMany: by every thread, the conditions are block-uniform
-            if (!nd_ok || done) continue;
+            q_ld(t, Q);
             double Fl[DIM][nV];
             PDE::template flux<DIM>(Q, Fl);
 #pragma unroll
@@ -391,8 +333,7 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
       }
       if (!reuse) __syncthreads();
       // C: rhs at this node, folded into the Picard accumulators
-      if (!nd_ok) {
-      } else if (!done && low) {  // increment: the rhs0 term cancels
+      if (!done && low) {  // increment: the rhs0 term cancels
         const int t = t0;
 #pragma unroll
         for (int v = 0; v < nV; v++) {
@@ -441,12 +382,11 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
     }
     // residual, reduced per cell by one warp
     double part = 0.0;
-    if (kTMany || !done) {
+    if (!done) {
 #pragma unroll
       for (int l = 0; l < b; l++) {
         double qo[nD];
         if (!low) q_ld(l, qo);
-        if (kTMany && done) continue;
 #pragma unroll
         for (int v = 0; v < nV; v++) {
           const double dq = low ? qn[l][v] : qn[l][v] - qo[v];
@@ -455,75 +395,25 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
         }
       }
     }
-    double sq_res;
-    if constexpr (TM && C::CPB == 1) {
-      // whole warps, one cell: each warp sums its lanes (the threads without
-      // a node add zero), one barrier, every thread adds the warp sums in
-      // the same order
-      constexpr int NW = C::THREADS / 32;
-      double acc = nd_ok ? part : 0.0;
+    sR[p] = part;
+    __syncthreads();
+    {
+      constexpr int kFullWarps = C::THREADS / 32;
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      if (warp < kFullWarps) {
+        for (int c = warp; c < C::CPB; c += kFullWarps) {
+          double* rr = smem + C::CPB * (C::SQ + C::SF) + c * C::SR;
+          double acc = 0.0;
+          for (int i = lane; i < P; i += 32) acc += rr[i];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if ((threadIdx.x & 31) == 0) sR[warp] = acc;
-      __syncthreads();
-      sq_res = 0.0;
-#pragma unroll
-      for (int w = 0; w < NW; w++) sq_res += sR[w];
-    } else {
-      if (nd_ok) sR[p] = part;
-      __syncthreads();
-      {
-        constexpr int kFullWarps = C::THREADS / 32;
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (warp < kFullWarps) {
-          for (int c = warp; c < C::CPB; c += kFullWarps) {
-            double* rr = smem + C::CPB * (C::SQ + C::SF) + c * C::SR;
-            double acc = 0.0;
-            for (int i = lane; i < P; i += 32) acc += rr[i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) rr[P] = acc;
-          }
+          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          if (lane == 0) rr[P] = acc;
         }
       }
-      __syncthreads();
-      sq_res = sR[P];
     }
-    if constexpr (kTMany) {
-      // every thread: each slice's old iterate is read and the new one (a
-      // finished cell: the old one) written back; a cell that converges now
-      // takes the time average of its old fluxes
-      const bool conv = !done && (sq_res < 1e-7 * 1e-7 || iter + 1 == C::maxIter);
-      if (!done) it_done = iter + 1;
-      double fh[DIM][nV];
-#pragma unroll
-      for (int d = 0; d < DIM; d++)
-#pragma unroll
-        for (int v = 0; v < nV; v++) fh[d][v] = 0.0;
-#pragma unroll
-      for (int t = 0; t < b; t++) {
-        double Q[nD], W[nD];
-        q_ld(t, Q);
-#pragma unroll
-        for (int v = 0; v < nD; v++) W[v] = done ? Q[v] : qn[t][v];
-        q_st(t, W);
-        if (conv && nd_ok) {
-          double Fl[DIM][nV];
-          PDE::template flux<DIM>(Q, Fl);
-#pragma unroll
-          for (int d = 0; d < DIM; d++)
-#pragma unroll
-            for (int v = 0; v < nV; v++) fh[d][v] += Fl[d][v] * T.w[t];
-        }
-      }
-      if (conv && nd_ok)
-#pragma unroll
-        for (int d = 0; d < DIM; d++)
-#pragma unroll
-          for (int v = 0; v < nV; v++) sF[sa[d] + v] = fh[d][v];
-      if (conv) done = true;
-      tmem::wait_st();
-    } else if (!done) {
+    __syncthreads();
+    const double sq_res = sR[P];
+    if (!done) {
       it_done = iter + 1;
       if (sq_res < 1e-7 * 1e-7 || iter + 1 == C::maxIter) {
         // time-averaged fluxes of this sweep = of the iterate before the
@@ -548,7 +438,6 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
           } else {
             q_st(t, qn[t]);
           }
-          if (!nd_ok) continue;
           double Fl[DIM][nV];
           PDE::template flux<DIM>(Q, Fl);
 #pragma unroll
@@ -563,11 +452,10 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
               for (int v = 0; v < nV; v++) dst[d * nV + v] = Fl[d][v];
           }
         }
-        if (nd_ok)
 #pragma unroll
-          for (int d = 0; d < DIM; d++)
+        for (int d = 0; d < DIM; d++)
 #pragma unroll
-            for (int v = 0; v < nV; v++) sF[sa[d] + v] = fh[d][v];
+          for (int v = 0; v < nV; v++) sF[sa[d] + v] = fh[d][v];
         done = true;
       } else {
 #pragma unroll
@@ -580,7 +468,6 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
           }
         }
       }
-      if (tm) tmem::wait_st();  // the next sweep (or the time average) reads them
     }
     if (p == 0) s_done[lc] = done;
     if constexpr (C::CPB == 1) {  // one cell: every thread read the same sum
@@ -616,16 +503,10 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
       fhd[(DIM * P + p) * nV + v] = 0.0;
     }
   }
-  if constexpr (TM) tmem::fence_before_sync();
   __syncthreads();
-  if constexpr (TM) {  // every warp has read its iterate (each load waited)
-    tmem::fence_after_sync();
-    if (warp == 0) tmem::dealloc(s_tbase, C::TCOLS);
-  }
   double* sQh = sQ;  // lQhi [P][nD]
 #pragma unroll
-  for (int v = 0; v < nD; v++)
-    if (nd_ok) sQh[p * nD + v] = qh[v];
+  for (int v = 0; v < nD; v++) sQh[p * nD + v] = qh[v];
   if (p == 0) s_done[lc] = !active;
   __syncthreads();
 
@@ -694,7 +575,7 @@ __global__ void __launch_bounds__(LinesCfg<DIM, N, PDE, MINB, MIXED, TS, TM>::TH
   // now) and written by consecutive threads to consecutive addresses: a
   // node's own nV doubles per thread would make every store instruction a
   // partial write of 32 sectors
-  if (active && nd_ok) {
+  if (active) {
 #pragma unroll
     for (int v = 0; v < nV; v++) {
       double du = 0.0;

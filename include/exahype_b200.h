@@ -85,9 +85,10 @@ int exa_solver_sizes(const exa_solver* s, int* sizes4);
  * (optional) receives the per-variant milliseconds. It allocates and frees
  * its own device buffers and synchronises the device. */
 #define EXA_PREDICTOR_VARIANTS 9  /* size of variant_ms; 4 and 5 (mixed) are not timed (-1) */
-/* Variant 8 keeps the Picard iterate of the line-form predictor in the SM's
- * tensor memory (solvers of order up to 5 with five state variables; other
- * shapes run variant 6 under this number). */
+/* Variant 8 keeps the Picard iterate in the SM's tensor memory (PDEs of five
+ * state variables without parameters and source terms; other shapes run
+ * variant 6 under this number). Variant 0, what a solver starts with, is the
+ * same form where variant 8 has it, the node form elsewhere. */
 /* Variants beyond the autotuned ones (exa_solver_set_variant only): the
  * mixed-precision predictor. Its first Picard sweep is the FP64 sweep; every
  * later sweep forms the flux increment F(q^k) - F(q^(k-1)) in FP64 and runs

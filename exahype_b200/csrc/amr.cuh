@@ -31,14 +31,16 @@
 
 namespace exa {
 
-// Operator tables in constant memory, packed over the orders 1..9 (offset of
-// order N: sum over lower orders of (N'+1)^2, times 3 for the thirds):
+// Operator tables in constant memory, packed over the orders that have kernels
+// (3, 4, 5 and 7; the offset of order N is the sum over the lower ones of
+// (N'+1)^2, times 3 for the thirds):
 // fineGridProjector1d [third][n][m], the restriction factors
 // w_n P[third][m][n] / (3 w_m) as [third][m][n], equidistantGridProjector1d
 // [n][i]. A block reads one matrix with block-uniform addresses, so the
 // coefficients come from the constant cache by broadcast.
-constexpr int amr_off(int N) { return N <= 1 ? 0 : amr_off(N - 1) + N * N; }
-constexpr int kAmrSq = amr_off(kMaxOrder + 1);  // sum of (N+1)^2 over N = 1..9
+constexpr bool amr_has(int N) { return N == 3 || N == 4 || N == 5 || N == 7; }
+constexpr int amr_off(int N) { return N <= 3 ? 0 : amr_off(N - 1) + (amr_has(N - 1) ? N * N : 0); }
+constexpr int kAmrSq = amr_off(8);  // sum of (N+1)^2 over the orders
 __constant__ double c_amr_fine[3 * kAmrSq];
 __constant__ double c_amr_restr[3 * kAmrSq];
 __constant__ double c_amr_equi[kAmrSq];

@@ -80,6 +80,16 @@ static void sfree(void* p, cudaStream_t st) {
 }
 
 // ---- tables ---------------------------------------------------------------
+template <int N>
+static void fill_proj_tables(ProjTables<N>& t) {
+  constexpr int b = N + 1, B = 2 * N + 1;
+  for (int i = 0; i < b * B; i++) {
+    t.uh2lim[i] = exa_tab_uh2lim[exa_tab_uh2lim_off[N] + i];
+    t.lim2uh[i] = exa_tab_lim2uh[exa_tab_lim2uh_off[N] + i];
+  }
+  for (int i = 0; i < b * b; i++) t.uh2lob[i] = exa_tab_uh2lob[exa_tab_uh2lob_off[N] + i];
+}
+
 static int upload_tables() {
   static std::mutex mu;
   static std::vector<int> done_dev;
@@ -89,15 +99,12 @@ static int upload_tables() {
   for (int d : done_dev)
     if (d == dev) return EXA_OK;
   std::vector<OrderTables> h(kMaxOrder + 1);
-  std::vector<LimiterTables> hl(kMaxOrder + 1);
   std::vector<double> afine(3 * kAmrSq, 0.0), arestr(3 * kAmrSq, 0.0), aequi(kAmrSq, 0.0);
   std::memset(h.data(), 0, sizeof(OrderTables) * h.size());
-  std::memset(hl.data(), 0, sizeof(LimiterTables) * hl.size());
 
   for (int N = 1; N <= kMaxOrder; N++) {
-    const int b = N + 1, bl = 2 * N + 1;
+    const int b = N + 1;
     OrderTables& t = h[N];
-    LimiterTables& l = hl[N];
     for (int i = 0; i < b; i++) {
       t.w[i] = exa_tab_weights[exa_tab_weights_off[N] + i];
       t.x[i] = exa_tab_nodes[exa_tab_nodes_off[N] + i];
@@ -110,7 +117,6 @@ static int upload_tables() {
       t.iK1[i] = exa_tab_iK1[exa_tab_iK1_off[N] + i];
       t.dudx[i] = exa_tab_dudx[exa_tab_dudx_off[N] + i];
       t.Kxi_f[i] = (float)t.Kxi[i];
-      l.uh2lob[i] = exa_tab_uh2lob[exa_tab_uh2lob_off[N] + i];
     }
     if (b % 2 == 0) {
       const int hh = b / 2;
@@ -120,10 +126,7 @@ static int upload_tables() {
           t.KxiQ[n * hh + m] = 0.5 * (t.Kxi[n * b + m] - t.Kxi[(b - 1 - n) * b + m]);
         }
     }
-    for (int i = 0; i < b * bl; i++) {
-      l.uh2lim[i] = exa_tab_uh2lim[exa_tab_uh2lim_off[N] + i];
-      l.lim2uh[i] = exa_tab_lim2uh[exa_tab_lim2uh_off[N] + i];
-    }
+    if (!amr_has(N)) continue;
     double* fine = afine.data() + 3 * amr_off(N);
     for (int i = 0; i < 3 * b * b; i++) fine[i] = exa_tab_fineGridProjector1d[exa_tab_fineGridProjector1d_off[N] + i];
     for (int j = 0; j < 3; j++)
@@ -140,7 +143,12 @@ static int upload_tables() {
   fill_line_tables(h[5], lt->n5);
   fill_line_tables(h[7], lt->n7);
   EXA_CUDA(cudaMemcpyToSymbol(c_line, lt.get(), sizeof(LineTablesAll)));
-  EXA_CUDA(cudaMemcpyToSymbol(g_lim_tab, hl.data(), sizeof(LimiterTables) * hl.size()));
+  std::unique_ptr<ProjTablesAll> pt(new ProjTablesAll());
+  fill_proj_tables(pt->n3);
+  fill_proj_tables(pt->n4);
+  fill_proj_tables(pt->n5);
+  fill_proj_tables(pt->n7);
+  EXA_CUDA(cudaMemcpyToSymbol(c_proj, pt.get(), sizeof(ProjTablesAll)));
   EXA_CUDA(cudaMemcpyToSymbol(c_amr_fine, afine.data(), sizeof(double) * afine.size()));
   EXA_CUDA(cudaMemcpyToSymbol(c_amr_restr, arestr.data(), sizeof(double) * arestr.size()));
   EXA_CUDA(cudaMemcpyToSymbol(c_amr_equi, aequi.data(), sizeof(double) * aequi.size()));

@@ -110,89 +110,121 @@ __device__ __forceinline__ void swap_group(double* __restrict__ a, double* __res
   }
 }
 
+// The 1-D projections of one order in constant memory: DG basis k -> subcell i
+// [k][i], subcell i -> DG basis j [i][j], DG basis j at Lobatto node i [j][i].
+template <int N>
+struct ProjTables {
+  static constexpr int b = N + 1, B = 2 * N + 1;
+  double uh2lim[b * B], lim2uh[B * b], uh2lob[b * b];
+};
+struct ProjTablesAll {
+  ProjTables<3> n3;
+  ProjTables<4> n4;
+  ProjTables<5> n5;
+  ProjTables<7> n7;
+};
+__constant__ ProjTablesAll c_proj;
+template <int N>
+__device__ __forceinline__ const ProjTables<N>& proj_tab() {
+  if constexpr (N == 3) return c_proj.n3;
+  else if constexpr (N == 4) return c_proj.n4;
+  else if constexpr (N == 5) return c_proj.n5;
+  else return c_proj.n7;
+}
+enum class Proj { kToFV, kToDG, kToLobatto };
+template <int N, Proj P>
+__device__ __forceinline__ const double* proj_matrix() {
+  return P == Proj::kToFV ? proj_tab<N>().uh2lim : P == Proj::kToDG ? proj_tab<N>().lim2uh : proj_tab<N>().uh2lob;
+}
+
+// Threads of a group that work on the lines of a tensor map: a multiple of the
+// five variables, so that a thread keeps one variable (tid % 5) throughout.
+template <class G>
+__device__ __forceinline__ int line_threads() { return G::size() / 5 * 5; }
+
+// out[o] = sum_i in[i] M[i][o] of one line, the matrix entries compile-time
+// constant-memory operands
+template <int IN, int OUT, class Out>
+__device__ __forceinline__ void map_line(const double (&in)[IN], const double* M, Out out) {
+#pragma unroll
+  for (int o = 0; o < OUT; o++) {
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < IN; i++) s += in[i] * M[i * OUT + o];
+    out(o, s);
+  }
+}
+
 // Separable tensor-product maps for one cell, executed by one thread group.
 // out[o1..][v] = sum_in src[in..][v] prod_d M[in_d][o_d], M row-major [IN][OUT].
 // Summation is per axis (x, then y, then z) rather than the reference's single
-// triple loop; the difference is at round-off level.
+// triple loop; the difference is at round-off level. A thread takes whole
+// lines: it loads a line's IN values once and forms all OUT of its outputs (per
+// output value each would load IN values and IN matrix entries, which made the
+// projections shared-memory bound: 729 patches 3D N=5 to subcells 38 -> 13 us,
+// a limiting step of 81^2 N=5 209 -> 195 us). Each loop over the lines stays a
+// loop: its body is already OUT chains wide. dst is called with the thread's own
+// variable, tid % 5.
 template <int DIM, int IN, int OUT, class G = BlockGroup, class Src, class Dst>
 __device__ void tensor_map(Src src, Dst dst, const double* M, double* tmp) {
   constexpr int nV = 5;
-  if constexpr (DIM == 2 && std::is_same<G, WarpGroup>::value) {
-    // one warp: a lane per (row, column) pair with the 5 variables unrolled,
-    // so that the index arithmetic is paid once per pair and dst sees a
-    // compile-time variable; every output is the same fma chain, in the same
-    // order, as in the generic form below
-    for (int i = G::tid(); i < IN * OUT; i += 32) {
-      const int xo = i % OUT, y = i / OUT;
-      double s[nV];
+  const int A = line_threads<G>(), tid = G::tid(), v = tid % nV;
+  if constexpr (DIM == 2) {
+    if (tid < A) {
+#pragma unroll 1
+      for (int l = tid; l < IN * nV; l += A) {  // t[y][xo][v], line (y, v)
+        const int y = l / nV;
+        double in[IN];
 #pragma unroll
-      for (int v = 0; v < nV; v++) s[v] = 0.0;
-#pragma unroll
-      for (int x = 0; x < IN; x++) {
-        const double m = M[x * OUT + xo];
-#pragma unroll
-        for (int v = 0; v < nV; v++) s[v] += src(0, y, x, v) * m;
+        for (int x = 0; x < IN; x++) in[x] = src(0, y, x, v);
+        map_line<IN, OUT>(in, M, [&](int xo, double s) { tmp[(y * OUT + xo) * nV + v] = s; });
       }
-#pragma unroll
-      for (int v = 0; v < nV; v++) tmp[i * nV + v] = s[v];
     }
     G::sync();
-    for (int i = G::tid(); i < OUT * OUT; i += 32) {
-      const int xo = i % OUT, yo = i / OUT;
-      double s[nV];
+    if (tid < A) {
+#pragma unroll 1
+      for (int l = tid; l < OUT * nV; l += A) {  // line (xo, v)
+        const int xo = l / nV;
+        double in[IN];
 #pragma unroll
-      for (int v = 0; v < nV; v++) s[v] = 0.0;
-#pragma unroll
-      for (int y = 0; y < IN; y++) {
-        const double m = M[y * OUT + yo];
-#pragma unroll
-        for (int v = 0; v < nV; v++) s[v] += tmp[(y * OUT + xo) * nV + v] * m;
+        for (int y = 0; y < IN; y++) in[y] = tmp[y * OUT * nV + l];
+        map_line<IN, OUT>(in, M, [&](int yo, double s) { dst(0, yo, xo, v, s); });
       }
-#pragma unroll
-      for (int v = 0; v < nV; v++) dst(0, yo, xo, v, s[v]);
-    }
-  } else if (DIM == 2) {
-    // t[y][xo][v] = sum_x src(y,x,v) M[x][xo]
-    for (int i = G::tid(); i < IN * OUT * nV; i += G::size()) {
-      const int v = i % nV, xo = (i / nV) % OUT, y = i / (nV * OUT);
-      double s = 0.0;
-#pragma unroll
-      for (int x = 0; x < IN; x++) s += src(0, y, x, v) * M[x * OUT + xo];
-      tmp[i] = s;
-    }
-    G::sync();
-    for (int i = G::tid(); i < OUT * OUT * nV; i += G::size()) {
-      const int v = i % nV, xo = (i / nV) % OUT, yo = i / (nV * OUT);
-      double s = 0.0;
-#pragma unroll
-      for (int y = 0; y < IN; y++) s += tmp[(y * OUT + xo) * nV + v] * M[y * OUT + yo];
-      dst(0, yo, xo, v, s);
     }
   } else {
-    double* t1 = tmp;                      // [z][y][xo]
-    double* t2 = tmp + IN * IN * OUT * nV;  // [z][yo][xo]
-    for (int i = G::tid(); i < IN * IN * OUT * nV; i += G::size()) {
-      const int v = i % nV, xo = (i / nV) % OUT, y = (i / (nV * OUT)) % IN, z = i / (nV * OUT * IN);
-      double s = 0.0;
+    double* t1 = tmp;                      // [z][y][xo][v]
+    double* t2 = tmp + IN * IN * OUT * nV;  // [z][yo][xo][v]
+    if (tid < A) {
+#pragma unroll 1
+      for (int l = tid; l < IN * IN * nV; l += A) {  // line (z, y, v)
+        const int zy = l / nV, z = zy / IN, y = zy - z * IN;
+        double in[IN];
 #pragma unroll
-      for (int x = 0; x < IN; x++) s += src(z, y, x, v) * M[x * OUT + xo];
-      t1[i] = s;
+        for (int x = 0; x < IN; x++) in[x] = src(z, y, x, v);
+        map_line<IN, OUT>(in, M, [&](int xo, double s) { t1[(zy * OUT + xo) * nV + v] = s; });
+      }
     }
     G::sync();
-    for (int i = G::tid(); i < IN * OUT * OUT * nV; i += G::size()) {
-      const int v = i % nV, xo = (i / nV) % OUT, yo = (i / (nV * OUT)) % OUT, z = i / (nV * OUT * OUT);
-      double s = 0.0;
+    if (tid < A) {
+#pragma unroll 1
+      for (int l = tid; l < IN * OUT * nV; l += A) {  // line (z, xo, v)
+        const int z = l / (OUT * nV), r = l - z * (OUT * nV);
+        double in[IN];
 #pragma unroll
-      for (int y = 0; y < IN; y++) s += t1[((z * IN + y) * OUT + xo) * nV + v] * M[y * OUT + yo];
-      t2[i] = s;
+        for (int y = 0; y < IN; y++) in[y] = t1[(z * IN + y) * OUT * nV + r];
+        map_line<IN, OUT>(in, M, [&](int yo, double s) { t2[(z * OUT + yo) * OUT * nV + r] = s; });
+      }
     }
     G::sync();
-    for (int i = G::tid(); i < OUT * OUT * OUT * nV; i += G::size()) {
-      const int v = i % nV, xo = (i / nV) % OUT, yo = (i / (nV * OUT)) % OUT, zo = i / (nV * OUT * OUT);
-      double s = 0.0;
+    if (tid < A) {
+#pragma unroll 1
+      for (int l = tid; l < OUT * OUT * nV; l += A) {  // line (yo, xo, v)
+        const int yx = l / nV, yo = yx / OUT, xo = yx - yo * OUT;
+        double in[IN];
 #pragma unroll
-      for (int z = 0; z < IN; z++) s += t2[((z * OUT + yo) * OUT + xo) * nV + v] * M[z * OUT + zo];
-      dst(zo, yo, xo, v, s);
+        for (int z = 0; z < IN; z++) in[z] = t2[z * OUT * OUT * nV + l];
+        map_line<IN, OUT>(in, M, [&](int zo, double s) { dst(zo, yo, xo, v, s); });
+      }
     }
   }
   G::sync();
@@ -205,12 +237,12 @@ constexpr int tensor_tmp() {
 
 // projectOnFVLimiterSpace (Limiter.cpp:23-66): DG nodes -> interior subcells
 template <int DIM, int N, class G = BlockGroup>
-__device__ void project_fv_block(const double* luh, double* lim, double* tmp, const double* uh2lim = nullptr) {
+__device__ void project_fv_block(const double* luh, double* lim, double* tmp) {
   using L = LimShape<DIM, N>;
   tensor_map<DIM, L::b, L::B, G>(
       [&](int z, int y, int x, int v) { return luh[(((DIM == 3 ? z * L::b : 0) + y) * L::b + x) * L::nV + v]; },
       [&](int z, int y, int x, int v, double s) { lim[lim_index<DIM, N>(z, y, x) * L::nV + v] = s; },
-      uh2lim ? uh2lim : g_lim_tab[N].uh2lim, tmp);
+      proj_matrix<N, Proj::kToFV>(), tmp);
 }
 // projectOnDGSpace (Limiter.cpp:69-112): interior subcells -> DG nodes
 template <int DIM, int N, class G = BlockGroup>
@@ -219,74 +251,68 @@ __device__ void project_dg_block(const double* lim, double* luh, double* tmp) {
   tensor_map<DIM, L::B, L::b, G>(
       [&](int z, int y, int x, int v) { return lim[lim_index<DIM, N>(z, y, x) * L::nV + v]; },
       [&](int z, int y, int x, int v, double s) { luh[(((DIM == 3 ? z * L::b : 0) + y) * L::b + x) * L::nV + v] = s; },
-      g_lim_tab[N].lim2uh, tmp);
+      proj_matrix<N, Proj::kToDG>(), tmp);
 }
 
-// block-wide min/max of 5 variables: each thread passes its partial values
-__device__ __forceinline__ void block_minmax5(double* mn, double* mx, double* red /*[2*5*32]*/) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int v = 0; v < 5; v++) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double a = __shfl_xor_sync(0xffffffffu, mn[v], o);
-      const double c = __shfl_xor_sync(0xffffffffu, mx[v], o);
-      mn[v] = (a < mn[v]) ? a : mn[v];
-      mx[v] = (mx[v] < c) ? c : mx[v];
-    }
-    if (lane == 0) {
-      red[v * 32 + warp] = mn[v];
-      red[160 + v * 32 + warp] = mx[v];
-    }
+// running minimum and maximum (a NaN never replaces them)
+struct MinMax {
+  double mn, mx;
+  __device__ __forceinline__ MinMax() : mn(1.7976931348623157e308), mx(-1.7976931348623157e308) {}  // DBL_MAX
+  __device__ __forceinline__ void fold(double lo, double hi) {
+    mn = (lo < mn) ? lo : mn;
+    mx = (mx < hi) ? hi : mx;
   }
-  __syncthreads();
-  if (warp == 0) {
+};
+
+// min/max per variable over a group whose thread tid < line_threads holds
+// those of variable tid % 5. One warp: lane v < 5 ends with variable v's
+// (lanes 5 apart hold the same variable: three exchanges).
+__device__ __forceinline__ MinMax warp_minmax_lines(MinMax m) {
+  if ((threadIdx.x & 31) >= 30) m = MinMax();
+#pragma unroll
+  for (int o : {15, 10, 5}) {
+    // (other lanes fold values of their own variable, or neutral ones)
+    const double lo = __shfl_down_sync(0xffffffffu, m.mn, o), hi = __shfl_down_sync(0xffffffffu, m.mx, o);
+    m.fold(lo, hi);
+  }
+  return m;
+}
+template <class G>
+struct GroupReduce {  // a whole block, through shared memory (red: 2 blockDim.x + 10): every thread ends with all five
+  __device__ static void minmax5(MinMax m, double* mn, double* mx, double* red) {
+    const int n = blockDim.x, A = line_threads<BlockGroup>();
+    red[threadIdx.x] = m.mn;
+    red[n + threadIdx.x] = m.mx;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      MinMax r;
+      if (threadIdx.x < 30)
+        for (int i = threadIdx.x; i < A; i += 30) r.fold(red[i], red[n + i]);
+      r = warp_minmax_lines(r);
+      if (threadIdx.x < 5) {
+        red[2 * n + threadIdx.x] = r.mn;
+        red[2 * n + 5 + threadIdx.x] = r.mx;
+      }
+    }
+    __syncthreads();
 #pragma unroll
     for (int v = 0; v < 5; v++) {
-      double a = lane < nw ? red[v * 32 + lane] : __longlong_as_double(0x7fefffffffffffffll);
-      double c = lane < nw ? red[160 + v * 32 + lane] : -__longlong_as_double(0x7fefffffffffffffll);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double a2 = __shfl_xor_sync(0xffffffffu, a, o);
-        const double c2 = __shfl_xor_sync(0xffffffffu, c, o);
-        a = (a2 < a) ? a2 : a;
-        c = (c < c2) ? c2 : c;
-      }
-      if (lane == 0) {
-        red[v * 32] = a;
-        red[160 + v * 32] = c;
-      }
+      mn[v] = red[2 * n + v];
+      mx[v] = red[2 * n + 5 + v];
     }
+    __syncthreads();
   }
-  __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 5; v++) {
-    mn[v] = red[v * 32];
-    mx[v] = red[160 + v * 32];
-  }
-  __syncthreads();
-}
-
-// the same for one warp: shuffles only, every lane ends with the result
-__device__ __forceinline__ void warp_minmax5(double* mn, double* mx) {
-#pragma unroll
-  for (int v = 0; v < 5; v++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double a = __shfl_xor_sync(0xffffffffu, mn[v], o);
-      const double c = __shfl_xor_sync(0xffffffffu, mx[v], o);
-      mn[v] = (a < mn[v]) ? a : mn[v];
-      mx[v] = (mx[v] < c) ? c : mx[v];
-    }
-}
-
-template <class G>
-struct GroupReduce {  // a whole block: through shared memory
-  __device__ static void minmax5(double* mn, double* mx, double* red) { block_minmax5(mn, mx, red); }
 };
 template <>
-struct GroupReduce<WarpGroup> {  // one warp: shuffles
-  __device__ static void minmax5(double* mn, double* mx, double*) { warp_minmax5(mn, mx); }
+struct GroupReduce<WarpGroup> {  // one warp: every lane ends with all five
+  __device__ static void minmax5(MinMax m, double* mn, double* mx, double*) {
+    m = warp_minmax_lines(m);
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+      mn[v] = __shfl_sync(0xffffffffu, m.mn, v);
+      mx[v] = __shfl_sync(0xffffffffu, m.mx, v);
+    }
+  }
 };
 
 // ---------------------------------------------------------------------------
@@ -765,15 +791,15 @@ struct PostCfg {
   static constexpr int TMP = tensor_tmp<DIM, L::b, L::B>() > tensor_tmp<DIM, L::b, L::b>()
                                  ? tensor_tmp<DIM, L::b, L::B>() : tensor_tmp<DIM, L::b, L::b>();
   static constexpr int THREADS = 128;
-  static constexpr size_t SMEM = sizeof(double) * (TMP + 320);
+  static constexpr size_t SMEM = sizeof(double) * (TMP + 2 * THREADS + 10);
   // the post-update kernel of 2D meshes runs one warp per cell, 4 per block
   static constexpr bool kWarp = DIM == 2;
   using Group = typename std::conditional<kWarp, WarpGroup, BlockGroup>::type;
   static constexpr int CELLS = kWarp ? THREADS / 32 : 1;
-  // per cell: tensor-map scratch, reduction slots, the staged DG solution and
-  // the two projection tables
-  static constexpr int STAGE = L::P * L::nV + L::b * L::b + L::b * L::B;
-  static constexpr int PER = TMP + 320 + STAGE;
+  // per cell: tensor-map scratch, reduction slots (a whole block's), the
+  // staged DG solution
+  static constexpr int RED = kWarp ? 0 : 2 * THREADS + 10;
+  static constexpr int PER = TMP + RED + L::P * L::nV;
   static constexpr size_t POST_SMEM = sizeof(double) * CELLS * PER;
 };
 
@@ -783,38 +809,19 @@ struct PostCfg {
 // compareWithADERDGSolutionAtFVSubcellCenters, Limiter.cpp:210-368). Block-wide;
 // every thread ends with the cell's values in mn/mx.
 template <int DIM, int N, class G = BlockGroup>
-__device__ void local_minmax_block(const double* u, double* mn, double* mx, double* tmp, double* red,
-                                   const double* uh2lob, const double* uh2lim) {
+__device__ void local_minmax_block(const double* u, double* mn, double* mx, double* tmp, double* red) {
   using L = LimShape<DIM, N>;
   constexpr int nV = L::nV;
-#pragma unroll
-  for (int v = 0; v < 5; v++) {
-    mn[v] = __longlong_as_double(0x7fefffffffffffffll);
-    mx[v] = -mn[v];
-  }
-  for (int p = G::tid(); p < L::P; p += G::size()) {
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      const double q = u[p * nV + v];
-      mn[v] = (q < mn[v]) ? q : mn[v];
-      mx[v] = (mx[v] < q) ? q : mx[v];
-    }
-  }
-  // the projected values are folded into the running min/max as they are
-  // produced; the variable is selected with compile-time indices so that
-  // mn/mx stay in registers
-  auto fold = [&](int, int, int, int v, double val) {
-#pragma unroll
-    for (int w = 0; w < 5; w++)
-      if (w == v) {
-        mn[w] = (val < mn[w]) ? val : mn[w];
-        mx[w] = (mx[w] < val) ? val : mx[w];
-      }
-  };
+  MinMax m;  // of this thread's variable
+  const int A = line_threads<G>();
+  if (G::tid() < A)
+    for (int e = G::tid(); e < L::P * nV; e += A) m.fold(u[e], u[e]);
+  // the projected values are folded in as they are produced
+  auto fold = [&](int, int, int, int, double val) { m.fold(val, val); };
   auto src = [&](int z, int y, int x, int v) { return u[(((DIM == 3 ? z * L::b : 0) + y) * L::b + x) * nV + v]; };
-  tensor_map<DIM, L::b, L::b, G>(src, fold, uh2lob, tmp);
-  tensor_map<DIM, L::b, L::B, G>(src, fold, uh2lim, tmp);
-  GroupReduce<G>::minmax5(mn, mx, red);
+  tensor_map<DIM, L::b, L::b, G>(src, fold, proj_matrix<N, Proj::kToLobatto>(), tmp);
+  tensor_map<DIM, L::b, L::B, G>(src, fold, proj_matrix<N, Proj::kToFV>(), tmp);
+  GroupReduce<G>::minmax5(m, mn, mx, red);
 }
 
 // Initial limiter status (updateLimiterStatusAndMinAndMaxAfterSetInitialConditions,
@@ -834,8 +841,7 @@ __global__ void __launch_bounds__(128) lim_init_kernel(int ncells, const double*
   const int cell = blockIdx.x;
   if (cell >= ncells) return;
   double mn[5], mx[5];
-  local_minmax_block<DIM, N>(luh + (size_t)cell * L::P * L::nV, mn, mx, smem, smem + C::TMP, g_lim_tab[N].uh2lob,
-                             g_lim_tab[N].uh2lim);
+  local_minmax_block<DIM, N>(luh + (size_t)cell * L::P * L::nV, mn, mx, smem, smem + C::TMP);
   if (threadIdx.x == 0) {
     double* mnB = minB + (size_t)cell * D2 * 5;
     double* mxB = maxB + (size_t)cell * D2 * 5;
@@ -904,9 +910,7 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
   extern __shared__ double smem[];
   double* tmp = smem + G::index() * C::PER;
   double* red = tmp + C::TMP;
-  double* su = red + 320;                  // the cell's DG solution after the update
-  double* slob = su + L::P * L::nV;        // uh2lob
-  double* slim = slob + L::b * L::b;       // uh2lim
+  double* su = red + C::RED;  // the cell's DG solution after the update
   __shared__ int s_flags_all[4][4];
   int* s_flags = s_flags_all[G::index()];
   const int cell = blockIdx.x * (blockDim.x / G::size()) + G::index();
@@ -941,17 +945,15 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
     G::sync();
     swap_group<G>(l, lp, L::LS);
     G::sync();
-    project_fv_block<DIM, N, G>(u, l, tmp, g_lim_tab[N].uh2lim);
+    project_fv_block<DIM, N, G>(u, l, tmp);
     if (G::tid() == 0) has_lim[cell] = 1;
   }
   if (st == 0 && G::tid() == 0) has_lim[cell] = 0;  // ensureNoUnrequiredLimiterPatchIsAllocatedOnComputeCell
   // admissible step of the new solution
   const double invDx0 = __ddiv_rn(1.0, geo.dx[0]), invDx1 = __ddiv_rn(1.0, geo.dx[1]);
   const double invDx2 = DIM == 3 ? __ddiv_rn(1.0, geo.dx[2]) : 0.0;
-  // stage the (final) DG solution and the projection tables of this order
+  // stage the (final) DG solution
   copy_group<G>(su, u, L::P * nV);
-  copy_group<G>(slob, g_lim_tab[N].uh2lob, L::b * L::b);
-  copy_group<G>(slim, g_lim_tab[N].uh2lim, L::b * L::B);
   G::sync();
   double dtm = __longlong_as_double(0x7fefffffffffffffll);
   for (int p = G::tid(); p < L::P; p += G::size()) {
@@ -973,26 +975,20 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
     if ((threadIdx.x & 31) == 0) atomic_min_pos_double(dt_min, m);
   }
   double mn[5], mx[5];
-  local_minmax_block<DIM, N, G>(su, mn, mx, tmp, red, slob, slim);
+  local_minmax_block<DIM, N, G>(su, mn, mx, tmp, red);
   // FV-subcell min/max of FV-active cells (findCellLocalLimiterMinAndMax, :167-205)
   double fmn[5], fmx[5];
   if (st >= prm.A) {
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      fmn[v] = __longlong_as_double(0x7fefffffffffffffll);
-      fmx[v] = -fmn[v];
-    }
+    MinMax m;  // of this thread's variable (a row holds B nV consecutive values)
+    const int A = line_threads<G>();
+    if (G::tid() < A)
 #pragma unroll 4
-    for (int i = G::tid(); i < L::PB; i += G::size()) {
-      const int x = i % L::B, y = (i / L::B) % L::B, z = DIM == 3 ? i / (L::B * L::B) : 0;
-      const double* q = l + lim_index<DIM, N>(z, y, x) * nV;
-#pragma unroll
-      for (int v = 0; v < 5; v++) {
-        fmn[v] = (q[v] < fmn[v]) ? q[v] : fmn[v];
-        fmx[v] = (fmx[v] < q[v]) ? q[v] : fmx[v];
+      for (int i = G::tid(); i < L::PB * nV; i += A) {
+        const int row = i / (L::B * nV), o = i - row * (L::B * nV);
+        const double q = l[lim_index<DIM, N>(row / L::B, row % L::B, 0) * nV + o];
+        m.fold(q, q);
       }
-    }
-    GroupReduce<G>::minmax5(fmn, fmx, red);
+    GroupReduce<G>::minmax5(m, fmn, fmx, red);
   }
   if constexpr (kWarp) {
     // the same as the block form below, lane v < 5 taking variable v
@@ -1118,7 +1114,7 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
   if (s_flags[2]) {  // newly allocated patch: zeroed; projection for helper cells
     for (int i = G::tid(); i < L::LS; i += G::size()) l[i] = lp[i] = 0.0;
     G::sync();
-    if (s_flags[1] < prm.A) project_fv_block<DIM, N, G>(su, l, tmp, slim);
+    if (s_flags[1] < prm.A) project_fv_block<DIM, N, G>(su, l, tmp);
   }
 }
 

@@ -277,43 +277,31 @@ __device__ __forceinline__ MinMax warp_minmax_lines(MinMax m) {
   }
   return m;
 }
-template <class G>
-struct GroupReduce {  // a whole block, through shared memory (red: 2 blockDim.x + 10): every thread ends with all five
-  __device__ static void minmax5(MinMax m, double* mn, double* mx, double* red) {
-    const int n = blockDim.x, A = line_threads<BlockGroup>();
-    red[threadIdx.x] = m.mn;
-    red[n + threadIdx.x] = m.mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      MinMax r;
-      if (threadIdx.x < 30)
-        for (int i = threadIdx.x; i < A; i += 30) r.fold(red[i], red[n + i]);
-      r = warp_minmax_lines(r);
-      if (threadIdx.x < 5) {
-        red[2 * n + threadIdx.x] = r.mn;
-        red[2 * n + 5 + threadIdx.x] = r.mx;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      mn[v] = red[2 * n + v];
-      mx[v] = red[2 * n + 5 + v];
-    }
-    __syncthreads();
-  }
-};
-template <>
-struct GroupReduce<WarpGroup> {  // one warp: every lane ends with all five
-  __device__ static void minmax5(MinMax m, double* mn, double* mx, double*) {
-    m = warp_minmax_lines(m);
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      mn[v] = __shfl_sync(0xffffffffu, m.mn, v);
-      mx[v] = __shfl_sync(0xffffffffu, m.mx, v);
+// The same over a whole block, through shared memory (red: 2 blockDim.x + 10
+// doubles): every thread ends with all five.
+__device__ __forceinline__ void block_minmax_lines(MinMax m, double* mn, double* mx, double* red) {
+  const int n = blockDim.x, A = line_threads<BlockGroup>();
+  red[threadIdx.x] = m.mn;
+  red[n + threadIdx.x] = m.mx;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    MinMax r;
+    if (threadIdx.x < 30)
+      for (int i = threadIdx.x; i < A; i += 30) r.fold(red[i], red[n + i]);
+    r = warp_minmax_lines(r);
+    if (threadIdx.x < 5) {
+      red[2 * n + threadIdx.x] = r.mn;
+      red[2 * n + 5 + threadIdx.x] = r.mx;
     }
   }
-};
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < 5; v++) {
+    mn[v] = red[2 * n + v];
+    mx[v] = red[2 * n + 5 + v];
+  }
+  __syncthreads();
+}
 
 // ---------------------------------------------------------------------------
 // Face merge (mergeSolutionMinMaxOnFace :1654-1690, mergeNeighboursLimiterStatus
@@ -426,7 +414,7 @@ __global__ void __launch_bounds__(128) lim_fv_halo_kernel(const int* __restrict_
 // update lim_prev <- lim (FiniteVolumesSolver::updateSolution,
 // FiniteVolumesSolver.cpp:662-715). In 2D (lim_muscl_kernel) the evolved
 // boundary states and the edge fluxes of the whole patch live in shared
-// memory; in 3D (lim_muscl3_kernel) those of one plane.
+// memory beside the patch itself; in 3D (lim_muscl3_kernel) those of one plane.
 template <int N>
 struct MusclCfg {
   using L = LimShape<2, N>;
@@ -435,9 +423,18 @@ struct MusclCfg {
   static constexpr int W = NR * 2 * 2 * L::nV;     // evolved wL/wR
   static constexpr int NE = (L::B + 1) * L::B;     // edges per direction
   static constexpr int FX = 2 * NE * L::nV;        // edge fluxes
-  static constexpr int TMP = tensor_tmp<2, L::B, L::b>();
-  static constexpr size_t SMEM = sizeof(double) * (W + FX + TMP);
-  static constexpr int THREADS = 256;
+  static constexpr int U = L::LS;                  // the patch
+  // a thread per edge of both directions (and per subcell of the ring, which
+  // are fewer): each phase is one round. A patch is a chain of three short
+  // phases, so what counts is how many are in flight: three blocks an SM up to
+  // N = 5 (81^2 N=5, about a tenth of the cells: 20.5 us with 256 threads and
+  // the neighbours read from global memory, 16.2 with two blocks, 13.5 with
+  // three); N = 7 spills at two (25^2, 40 limiting steps 4.75 ms, with one 4.50).
+  static constexpr int THREADS = (2 * NE + 31) / 32 * 32;
+  static constexpr int MINB = THREADS <= 320 ? 3 : 1;
+  static constexpr size_t SMEM = sizeof(double) * (U + W + FX);
+  static_assert(NR <= THREADS, "one subcell of the ring per thread");
+  static_assert(tensor_tmp<2, L::B, L::b>() <= W, "the projection's scratch takes the states' place");
 };
 
 __device__ __forceinline__ double minmod_dev(double a, double b) {  // musclhancock.cpph:29-38
@@ -477,19 +474,18 @@ __device__ __forceinline__ void edge_flux(const double* ql, const double* qr, in
 }
 
 template <int N, class PDE>
-__global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ list, const int* __restrict__ count,
-                                                       int nlist, double* __restrict__ lim, double* __restrict__ lim_prev,
-                                                       double* __restrict__ luh, Geometry geo,
-                                                       const double* __restrict__ dt_ptr,
-                                                       const int* __restrict__ gate) {
+__global__ void __launch_bounds__(MusclCfg<N>::THREADS, MusclCfg<N>::MINB)
+    lim_muscl_kernel(const int* __restrict__ list, const int* __restrict__ count, int nlist, double* __restrict__ lim,
+                     double* __restrict__ lim_prev, double* __restrict__ luh, Geometry geo,
+                     const double* __restrict__ dt_ptr, const int* __restrict__ gate) {
   constexpr int DIM = 2;
   using L = LimShape<2, N>;
   using C = MusclCfg<N>;
   constexpr int E = L::E, B = L::B, nV = L::nV, R = C::R;
   if (gate && !*gate) return;
   extern __shared__ double smem[];
-  double* tmp = smem;
-  double* W = smem + C::TMP;
+  double* sU = smem;  // the patch: read once from global memory
+  double* W = sU + C::U;
   double* FX = W + C::W;
   const double dt = *dt_ptr;
   double cs[DIM], ics[DIM], icsdt[DIM];
@@ -503,11 +499,12 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
     const int cell = list ? list[li] : li;
     double* l = lim + (size_t)cell * L::LS;
     double* lp = lim_prev + (size_t)cell * L::LS;
-    for (int i = threadIdx.x; i < L::LS; i += blockDim.x) lp[i] = l[i];
+    for (int i = threadIdx.x; i < L::LS; i += C::THREADS) lp[i] = sU[i] = l[i];
     __syncthreads();
-    auto U = [&](int y, int x, int v) { return lp[(y * E + x) * nV + v]; };
+    auto U = [&](int y, int x, int v) { return sU[(y * E + x) * nV + v]; };
     // slopes, extrapolation and half-step evolution on interior + first ghost ring
-    for (int q = threadIdx.x; q < C::NR; q += blockDim.x) {
+    if (threadIdx.x < C::NR) {
+      const int q = threadIdx.x;
       const int x = q % R + kGW - 1, y = q / R + kGW - 1;
       double wl[DIM][5], wr[DIM][5];
 #pragma unroll
@@ -534,54 +531,55 @@ __global__ void __launch_bounds__(256) lim_muscl_kernel(const int* __restrict__ 
 #pragma unroll
       for (int d = 0; d < DIM; d++)
 #pragma unroll
-        for (int v = 0; v < nV; v++) {
-          W[((q * DIM + d) * 2 + 0) * nV + v] = wl[d][v] + 0.5 * dt * Qt[v];
-          W[((q * DIM + d) * 2 + 1) * nV + v] = wr[d][v] + 0.5 * dt * Qt[v];
+        for (int v = 0; v < nV; v++) {  // [d][left, right][v][subcell]: consecutive threads, consecutive banks
+          W[((d * 2 + 0) * nV + v) * C::NR + q] = wl[d][v] + 0.5 * dt * Qt[v];
+          W[((d * 2 + 1) * nV + v) * C::NR + q] = wr[d][v] + 0.5 * dt * Qt[v];
         }
     }
     __syncthreads();
     // Rusanov flux on every subcell edge: edge e of direction d
     // joins positions k and k+1 along d, k in [-1, B) relative to the interior
-    for (int i = threadIdx.x; i < DIM * C::NE; i += blockDim.x) {
-      const int d = i / C::NE, e = i % C::NE;
+    if (threadIdx.x < DIM * C::NE) {
+      const int i = threadIdx.x, d = i / C::NE, e = i % C::NE;
       const int kk = e % (B + 1), t = e / (B + 1);  // position k + 1 along d, transverse interior coordinate
       const int qL = d == 0 ? (t + 1) * R + kk : kk * R + t + 1;  // ring index 0 = first ghost layer
       const int qR = qL + (d == 0 ? 1 : R);
-      const double* ql = W + ((qL * DIM + d) * 2 + 1) * nV;  // wR of the left subcell
-      const double* qr = W + ((qR * DIM + d) * 2 + 0) * nV;  // wL of the right subcell
-      double f[5];
+      double ql[5], qr[5], f[5];  // wR of the left subcell, wL of the right subcell
+#pragma unroll
+      for (int v = 0; v < nV; v++) {
+        ql[v] = W[((d * 2 + 1) * nV + v) * C::NR + qL];
+        qr[v] = W[((d * 2 + 0) * nV + v) * C::NR + qR];
+      }
       edge_flux<DIM, PDE>(ql, qr, d, f);
 #pragma unroll
       for (int v = 0; v < nV; v++) FX[i * nV + v] = f[v];
     }
     __syncthreads();
     // update of the interior subcells in the reference's accumulation order:
-    // +left x edge, -right x edge, then y, then z
-    for (int i = threadIdx.x; i < L::PB * nV; i += blockDim.x) {
+    // +left x edge, -right x edge, then y
+    for (int i = threadIdx.x; i < L::PB * nV; i += C::THREADS) {
       const int v = i % nV, sc = i / nV;
       const int x = sc % B, y = sc / B;
-      double u = U(y + kGW, x + kGW, v);
+      const int at = lim_index<2, N>(0, y, x) * nV + v;
+      double u = sU[at];
       // edge index within direction d: (transverse t, k) with k = position + 1 for the left edge
       u += icsdt[0] * FX[(y * (B + 1) + x) * nV + v];
       u -= icsdt[0] * FX[(y * (B + 1) + x + 1) * nV + v];
       u += icsdt[1] * FX[(C::NE + x * (B + 1) + y) * nV + v];
       u -= icsdt[1] * FX[(C::NE + x * (B + 1) + y + 1) * nV + v];
-      l[lim_index<2, N>(0, y, x) * nV + v] = u;
+      sU[at] = l[at] = u;
     }
     // the reference's edge loops also touch the first ghost layer on every
     // face (one edge each); the ghost corners stay untouched
-    for (int i = threadIdx.x; i < DIM * 2 * B * nV; i += blockDim.x) {
+    for (int i = threadIdx.x; i < DIM * 2 * B * nV; i += C::THREADS) {
       const int v = i % nV, t = (i / nV) % B, side = (i / (nV * B)) % 2, d = i / (nV * B * 2);
       const int c = t + kGW, k = side ? B + kGW : kGW - 1;
-      const int idx = d == 0 ? c * E + k : k * E + c;
+      const int at = (d == 0 ? c * E + k : k * E + c) * nV + v;
       const double f = FX[((d * C::NE) + t * (B + 1) + (side ? B : 0)) * nV + v];
-      if (side)
-        l[idx * nV + v] += icsdt[d] * f;
-      else
-        l[idx * nV + v] -= icsdt[d] * f;
+      l[at] = side ? sU[at] + icsdt[d] * f : sU[at] - icsdt[d] * f;
     }
     __syncthreads();
-    if (luh) project_dg_block<2, N>(l, luh + (size_t)cell * L::P * nV, tmp);
+    if (luh) project_dg_block<2, N>(sU, luh + (size_t)cell * L::P * nV, W);  // (ends with a barrier)
   }
 }
 
@@ -796,6 +794,7 @@ struct PostCfg {
   static constexpr bool kWarp = DIM == 2;
   using Group = typename std::conditional<kWarp, WarpGroup, BlockGroup>::type;
   static constexpr int CELLS = kWarp ? THREADS / 32 : 1;
+  static constexpr int BLOCKS = !kWarp ? 1 : N == 7 ? 5 : 8;  // per SM, of the post-update kernel's registers
   // per cell: tensor-map scratch, reduction slots (a whole block's), the
   // staged DG solution
   static constexpr int RED = kWarp ? 0 : 2 * THREADS + 10;
@@ -809,7 +808,7 @@ struct PostCfg {
 // compareWithADERDGSolutionAtFVSubcellCenters, Limiter.cpp:210-368). Block-wide;
 // every thread ends with the cell's values in mn/mx.
 template <int DIM, int N, class G = BlockGroup>
-__device__ void local_minmax_block(const double* u, double* mn, double* mx, double* tmp, double* red) {
+__device__ MinMax local_minmax_lines(const double* u, double* tmp) {
   using L = LimShape<DIM, N>;
   constexpr int nV = L::nV;
   MinMax m;  // of this thread's variable
@@ -821,7 +820,7 @@ __device__ void local_minmax_block(const double* u, double* mn, double* mx, doub
   auto src = [&](int z, int y, int x, int v) { return u[(((DIM == 3 ? z * L::b : 0) + y) * L::b + x) * nV + v]; };
   tensor_map<DIM, L::b, L::b, G>(src, fold, proj_matrix<N, Proj::kToLobatto>(), tmp);
   tensor_map<DIM, L::b, L::B, G>(src, fold, proj_matrix<N, Proj::kToFV>(), tmp);
-  GroupReduce<G>::minmax5(m, mn, mx, red);
+  return m;
 }
 
 // Initial limiter status (updateLimiterStatusAndMinAndMaxAfterSetInitialConditions,
@@ -841,7 +840,7 @@ __global__ void __launch_bounds__(128) lim_init_kernel(int ncells, const double*
   const int cell = blockIdx.x;
   if (cell >= ncells) return;
   double mn[5], mx[5];
-  local_minmax_block<DIM, N>(luh + (size_t)cell * L::P * L::nV, mn, mx, smem, smem + C::TMP);
+  block_minmax_lines(local_minmax_lines<DIM, N>(luh + (size_t)cell * L::P * L::nV, smem), mn, mx, smem + C::TMP);
   if (threadIdx.x == 0) {
     double* mnB = minB + (size_t)cell * D2 * 5;
     double* mxB = maxB + (size_t)cell * D2 * 5;
@@ -896,9 +895,12 @@ __global__ void __launch_bounds__(128) lim_seed_kernel(int ncells, const int* __
 //   - an irregular change (a cell with s <= A became troubled) sets *irregular.
 // run (optional): the kernel does nothing when it holds 0.
 // G: one block per cell (BlockGroup) or one warp per cell, 4 cells per block
-// (WarpGroup; 2D).
+// (WarpGroup; 2D). A warp is a chain of some ten dependent phases, so its
+// register budget is that of eight blocks an SM (81^2 N=5: all but 1.4 waves
+// of warps in flight; 48 limiting steps 7.15 ms, with six 7.23, five 7.24);
+// five at N = 7 (61^2, 40 steps: 6.93, with eight 6.99).
 template <int DIM, int N, class PDE, class G = BlockGroup>
-__global__ void __launch_bounds__(128) lim_post_update_kernel(
+__global__ void __launch_bounds__(128, PostCfg<DIM, N>::BLOCKS) lim_post_update_kernel(
     int ncells, double* __restrict__ luh, int* __restrict__ s, int* __restrict__ s_prev, int* __restrict__ cure,
     int* __restrict__ fs, int* __restrict__ has_lim, double* __restrict__ minB, double* __restrict__ maxB,
     double* __restrict__ lim, double* __restrict__ lim_prev, Geometry geo, LimParams prm,
@@ -974,42 +976,25 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
     }
     if ((threadIdx.x & 31) == 0) atomic_min_pos_double(dt_min, m);
   }
-  double mn[5], mx[5];
-  local_minmax_block<DIM, N, G>(su, mn, mx, tmp, red);
+  const MinMax dgm = local_minmax_lines<DIM, N, G>(su, tmp);
   // FV-subcell min/max of FV-active cells (findCellLocalLimiterMinAndMax, :167-205)
-  double fmn[5], fmx[5];
+  MinMax fvm;  // of this thread's variable (a row holds B nV consecutive values)
   if (st >= prm.A) {
-    MinMax m;  // of this thread's variable (a row holds B nV consecutive values)
     const int A = line_threads<G>();
     if (G::tid() < A)
 #pragma unroll 4
       for (int i = G::tid(); i < L::PB * nV; i += A) {
         const int row = i / (L::B * nV), o = i - row * (L::B * nV);
         const double q = l[lim_index<DIM, N>(row / L::B, row % L::B, 0) * nV + o];
-        m.fold(q, q);
+        fvm.fold(q, q);
       }
-    GroupReduce<G>::minmax5(m, fmn, fmx, red);
   }
   if constexpr (kWarp) {
     // the same as the block form below, lane v < 5 taking variable v
     const int lane = G::tid(), v = lane % 5;
-    double mnv = mn[0], mxv = mx[0], fmnv = 0.0, fmxv = 0.0;
-#pragma unroll
-    for (int w = 1; w < 5; w++)
-      if (w == v) {
-        mnv = mn[w];
-        mxv = mx[w];
-      }
-    if (st >= prm.A) {
-      fmnv = fmn[0];
-      fmxv = fmx[0];
-#pragma unroll
-      for (int w = 1; w < 5; w++)
-        if (w == v) {
-          fmnv = fmn[w];
-          fmxv = fmx[w];
-        }
-    }
+    const MinMax dr = warp_minmax_lines(dgm), fr = warp_minmax_lines(fvm);
+    const double mnv = __shfl_sync(0xffffffffu, dr.mn, v), mxv = __shfl_sync(0xffffffffu, dr.mx, v);
+    const double fmnv = __shfl_sync(0xffffffffu, fr.mn, v), fmxv = __shfl_sync(0xffffffffu, fr.mx, v);
     // discreteMaximumPrincipleAndMinAndMaxSearch (Limiter.cpp:114-165)
     double bmin = __shfl_sync(0xffffffffu, pmn, v), bmax = __shfl_sync(0xffffffffu, pmx, v);
 #pragma unroll
@@ -1022,7 +1007,15 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
     sd = (sd < prm.relax) ? prm.relax : sd;
     const bool okv = !((mnv < (bmin - sd)) || (mxv > (bmax + sd)));
     bool ok = __all_sync(0xffffffffu, lane >= 5 || okv);
-    if (ok) ok = PDE::isPhysicallyAdmissible(mn, mx);  // on the new local min/max
+    {
+      double mn[5], mx[5];
+#pragma unroll
+      for (int w = 0; w < 5; w++) {
+        mn[w] = __shfl_sync(0xffffffffu, mnv, w);
+        mx[w] = __shfl_sync(0xffffffffu, mxv, w);
+      }
+      if (ok) ok = PDE::isPhysicallyAdmissible(mn, mx);  // on the new local min/max
+    }
     double* mnB = minB + (size_t)cell * D2 * 5;
     double* mxB = maxB + (size_t)cell * D2 * 5;
     if (st >= prm.A) {
@@ -1063,52 +1056,57 @@ __global__ void __launch_bounds__(128) lim_post_update_kernel(
       s_flags[2] = (ns > 0 && !had);
       if (s_flags[2]) has_lim[cell] = 1;
     }
-  } else if (G::tid() == 0) {
-    double* mnB = minB + (size_t)cell * D2 * 5;
-    double* mxB = maxB + (size_t)cell * D2 * 5;
-    // discreteMaximumPrincipleAndMinAndMaxSearch (Limiter.cpp:114-165)
-    bool ok = true;
-    for (int v = 0; v < 5; v++) {
-      double bmin = mnB[v], bmax = mxB[v];
-      for (int i = 1; i < D2; i++) bmin = (mnB[i * 5 + v] < bmin) ? mnB[i * 5 + v] : bmin;
-      for (int i = 1; i < D2; i++) bmax = (bmax < mxB[i * 5 + v]) ? mxB[i * 5 + v] : bmax;
-      double sd = (bmax - bmin) * prm.scale;
-      sd = (sd < prm.relax) ? prm.relax : sd;
-      if ((mn[v] < (bmin - sd)) || (mx[v] > (bmax + sd))) ok = false;
-      mnB[v] = mn[v];
-      mxB[v] = mx[v];
-      mnB[v + 5] = bmin;
-      mxB[v + 5] = bmax;
-    }
-    if (ok) ok = PDE::isPhysicallyAdmissible(mnB, mxB);  // on the new local min/max
-    if (st >= prm.A)
-      for (int i = 0; i < D2; i++)
-        for (int v = 0; v < 5; v++) {
-          mnB[i * 5 + v] = fmn[v];
-          mxB[i * 5 + v] = fmx[v];
-        }
-    int ns;
-    if (!ok) {
-      cure[cell] = prm.cure_steps + 1;
-      if (!(st > prm.A)) atomicOr(irregular, 1);
-      ns = prm.T;
-    } else if (st >= prm.T) {
-      ns = prm.T;
-      cure[cell] -= 1;
-      if (cure[cell] == 0) {
-        ns = prm.T - 1;
-        cure[cell] = prm.cure_steps + 1;
+  } else {
+    double mn[5], mx[5], fmn[5], fmx[5];
+    block_minmax_lines(dgm, mn, mx, red);
+    if (st >= prm.A) block_minmax_lines(fvm, fmn, fmx, red);
+    if (G::tid() == 0) {
+      double* mnB = minB + (size_t)cell * D2 * 5;
+      double* mxB = maxB + (size_t)cell * D2 * 5;
+      // discreteMaximumPrincipleAndMinAndMaxSearch (Limiter.cpp:114-165)
+      bool ok = true;
+      for (int v = 0; v < 5; v++) {
+        double bmin = mnB[v], bmax = mxB[v];
+        for (int i = 1; i < D2; i++) bmin = (mnB[i * 5 + v] < bmin) ? mnB[i * 5 + v] : bmin;
+        for (int i = 1; i < D2; i++) bmax = (bmax < mxB[i * 5 + v]) ? mxB[i * 5 + v] : bmax;
+        double sd = (bmax - bmin) * prm.scale;
+        sd = (sd < prm.relax) ? prm.relax : sd;
+        if ((mn[v] < (bmin - sd)) || (mx[v] > (bmax + sd))) ok = false;
+        mnB[v] = mn[v];
+        mxB[v] = mx[v];
+        mnB[v + 5] = bmin;
+        mxB[v + 5] = bmax;
       }
-    } else {
-      ns = 0;
-      for (int i = 0; i < D2; i++) ns = max(ns, fs[cell * D2 + i]);
+      if (ok) ok = PDE::isPhysicallyAdmissible(mnB, mxB);  // on the new local min/max
+      if (st >= prm.A)
+        for (int i = 0; i < D2; i++)
+          for (int v = 0; v < 5; v++) {
+            mnB[i * 5 + v] = fmn[v];
+            mxB[i * 5 + v] = fmx[v];
+          }
+      int ns;
+      if (!ok) {
+        cure[cell] = prm.cure_steps + 1;
+        if (!(st > prm.A)) atomicOr(irregular, 1);
+        ns = prm.T;
+      } else if (st >= prm.T) {
+        ns = prm.T;
+        cure[cell] -= 1;
+        if (cure[cell] == 0) {
+          ns = prm.T - 1;
+          cure[cell] = prm.cure_steps + 1;
+        }
+      } else {
+        ns = 0;
+        for (int i = 0; i < D2; i++) ns = max(ns, fs[cell * D2 + i]);
+      }
+      s[cell] = ns;
+      for (int i = 0; i < D2; i++) fs[cell * D2 + i] = 0;
+      const int had = (st == 0) ? 0 : (st < prm.A ? 1 : has_lim[cell]);
+      s_flags[1] = ns;
+      s_flags[2] = (ns > 0 && !had);
+      if (s_flags[2]) has_lim[cell] = 1;
     }
-    s[cell] = ns;
-    for (int i = 0; i < D2; i++) fs[cell * D2 + i] = 0;
-    const int had = (st == 0) ? 0 : (st < prm.A ? 1 : has_lim[cell]);
-    s_flags[1] = ns;
-    s_flags[2] = (ns > 0 && !had);
-    if (s_flags[2]) has_lim[cell] = 1;
   }
   G::sync();
   if (s_flags[2]) {  // newly allocated patch: zeroed; projection for helper cells

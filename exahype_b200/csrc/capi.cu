@@ -314,18 +314,19 @@ struct Launch {
     else return false;
   }
   static constexpr bool kTmem = tmem_fits();
+  template <bool FEW>
   static int launch_tmem(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
                          Geometry g, int n, const int* list, const int* cnt, unsigned long long* acc,
                          cudaStream_t st) {
     if constexpr (kTmem) {
-      using TC = TmemCfg<DIM, N, PDE>;
+      using TC = TmemCfg<DIM, N, PDE, FEW>;
       static bool attr = false;
       if (!attr) {
-        EXA_CUDA(cudaFuncSetAttribute(predictor_tmem_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)TC::SMEM));
+        EXA_CUDA(cudaFuncSetAttribute(predictor_tmem_kernel<DIM, N, PDE, FEW>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC::SMEM));
         attr = true;
       }
-      predictor_tmem_kernel<DIM, N, PDE><<<(n + TC::CPB - 1) / TC::CPB, TC::THREADS, TC::SMEM, st>>>(
+      predictor_tmem_kernel<DIM, N, PDE, FEW><<<(n + TC::CPB - 1) / TC::CPB, TC::THREADS, TC::SMEM, st>>>(
           luh, qb, fb, du, iters, acc, dt, g, n, list, cnt);
       EXA_LAUNCHED();
     }
@@ -336,8 +337,13 @@ struct Launch {
                        Geometry g, int n, const int* list, const int* cnt, PredictorTemps tmp, bool temps,
                        unsigned long long* acc, int variant, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    if (kTmem && !temps && (variant == 0 || variant == 8))  // (counts its sweeps itself)
-      return launch_tmem(luh, qb, fb, du, iters, dt, g, n, list, cnt, acc, st);
+    if constexpr (kTmem)  // (counts its sweeps itself)
+      if (!temps && (variant == 0 || variant == 8)) {
+        using TC = TmemCfg<DIM, N, PDE>;
+        return n <= TC::kFewCells
+                   ? launch_tmem<(TC::kFewCells > 0)>(luh, qb, fb, du, iters, dt, g, n, list, cnt, acc, st)
+                   : launch_tmem<false>(luh, qb, fb, du, iters, dt, g, n, list, cnt, acc, st);
+      }
     int rc;
     if constexpr (PDE::kSource || PDE::kNCP)  // source terms: the node form (1 or 2 blocks per SM)
       rc = temps ? launch_pred<true, 1, 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st)

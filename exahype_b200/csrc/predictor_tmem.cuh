@@ -49,12 +49,26 @@
 
 namespace exa {
 
-template <int DIM, int N, class PDE>
+// Cells per block: what fits 128 threads (one warp for each quadrant of the
+// tensor memory's lanes), or one cell. A block waits at its barriers for all of
+// its cells and sweeps as often as the slowest, so smaller is better, as long as
+// the register file (512 threads of 128 registers) stays full: against blocks of
+// up to 256 threads 3D N=4 17,714 cells 474 -> 369 us, 3D N=3 31,868 cells
+// 361 -> 317, 2D N=7 13,176 cells 230 -> 191, 2D N=3 53,144 cells 124 -> 110,
+// 2D N=5 29,160 cells 197 -> 193 (the last warp of 128 is a third empty there).
+// FEW: so few cells that the chip is not full anyway (kFewCells). One cell per
+// block (two where they share a warp) spreads them over the SMs, and with no
+// budget for other blocks nothing spills: 81 cells 2D N=3 9.9 -> 9.6 us, N=4
+// 12.2 -> 10.4, N=7 17.6 -> 13.5, 216 cells 3D N=5 33.4 -> 31.5; at 729 cells
+// 2D N=4 takes 13.4 instead of 12.5 us.
+template <int DIM, int N, class PDE, bool FEW = false>
 struct TmemCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
-  static constexpr int CPB = cells_per_block<S::P>();
+  static constexpr int CPB = FEW ? (S::P == 16 ? 2 : 1) : S::P <= 128 ? 128 / S::P : 1;
   static constexpr int THREADS = (CPB * S::P + 31) / 32 * 32;
-  static constexpr int MINB = THREADS <= 256 ? 2 : 1;  // blocks per SM of the register budget
+  static constexpr int MINB = FEW ? 1 : 512 / THREADS;  // blocks per SM of the register budget
+  // cells up to which FEW is taken: two per SM
+  static constexpr int kFewCells = S::P < 512 ? 2 * 148 : 0;  // (3D N=7: the same block)
   static constexpr int LINES = S::F, LI = LINES * S::nV;
   static constexpr bool kByDir = LI <= S::P;
   static constexpr int ROUNDS = kByDir ? DIM : (DIM * LI + S::P - 1) / S::P;
@@ -83,13 +97,13 @@ struct TmemCfg : Shape<DIM, N, PDE> {
   static_assert(kByDir || sstride(0) == sstride(DIM - 1), "items over all directions: one stride");
 };
 
-template <int DIM, int N, class PDE>
-__global__ void __launch_bounds__(TmemCfg<DIM, N, PDE>::THREADS, TmemCfg<DIM, N, PDE>::MINB)
+template <int DIM, int N, class PDE, bool FEW>
+__global__ void __launch_bounds__(TmemCfg<DIM, N, PDE, FEW>::THREADS, TmemCfg<DIM, N, PDE, FEW>::MINB)
     predictor_tmem_kernel(const double* __restrict__ luh, double* __restrict__ lQhbnd, double* __restrict__ lFhbnd,
                           double* __restrict__ lduh, int* __restrict__ iters, unsigned long long* __restrict__ sweeps,
                           const double* __restrict__ dt_ptr, Geometry geo, int ncells,
                           const int* __restrict__ cell_list, const int* __restrict__ count) {
-  using C = TmemCfg<DIM, N, PDE>;
+  using C = TmemCfg<DIM, N, PDE, FEW>;
   constexpr int b = C::b, P = C::P, nV = C::nV, LI = C::LI, CPB = C::CPB, TS = C::TS;
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ double smem[];

@@ -2,7 +2,8 @@
 cells of one block, or of one warp, need different numbers of sweeps: constant
 states (one sweep) beside smooth ones, a cell whose state is not a number (all
 sweeps, and none of its neighbours' results may change), one cell alone, blocks
-that are not full, a permuted list. Sweep counts equal to the oracle's, arrays
+that are not full, a permuted list, counts on either side of the line between
+the blocks for few cells and the others (296). Sweep counts equal to the oracle's, arrays
 to 1e-12 of their largest entry (test_gpu_aderdg's FP64 bound)."""
 import numpy as np
 import pytest
@@ -23,7 +24,7 @@ def eb():
 
 
 @pytest.mark.parametrize("variant", [0, 8])
-@pytest.mark.parametrize("n", [1, 7, 19])
+@pytest.mark.parametrize("n", [1, 7, 296, 331])
 @pytest.mark.parametrize("dim,order", [(2, 3), (2, 4), (2, 5), (2, 7), (3, 3), (3, 4), (3, 5), (3, 7)])
 def test_mixed_sweep_counts_vs_oracle(eb, dim, order, n, variant):
     rng = np.random.default_rng(100 * dim + 10 * order + n)
@@ -49,7 +50,7 @@ def test_mixed_sweep_counts_vs_oracle(eb, dim, order, n, variant):
     torch.cuda.synchronize()
     qb, fb, du, it = (t.cpu().numpy() for t in (*out, du, it))
     k = pyoracle.Kernels(dim, order, pde=0)
-    for c in range(n):
+    for c in range(n) if n < 20 else [0, 1, 2, 3, 4, 5, 6, 7, n // 2, n - 3, n - 2, n - 1]:
         if c == bad:
             assert np.isnan(du[c]).any()
             continue

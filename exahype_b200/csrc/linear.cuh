@@ -50,7 +50,10 @@ struct GradPairs {
 template <int DIM, int N, class PDE>
 struct CKCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
-  static constexpr int CPB = cells_per_block<S::P>();
+  // what fits 128 threads, or one cell: a barrier joins fewer warps than in
+  // blocks of up to 256 threads (9,975 cells 3D N=4 232 -> 206 us, 19,683 cells
+  // N=3 218 -> 207, 6,561 cells 2D N=5 48 -> 44)
+  static constexpr int CPB = S::P <= 128 ? 128 / S::P : 1;
   static constexpr int THREADS = CPB * S::P;
   static constexpr int LINES = S::F;                                             // lines per direction
   static constexpr int NPAIRS = GradPairs<PDE, DIM>().n, NU = NPAIRS / DIM;  // gradient components, per direction
@@ -63,11 +66,10 @@ struct CKCfg : Shape<DIM, N, PDE> {
   // gradient items per thread; with NU == b one direction per round
   static constexpr int ROUNDS = (NPAIRS + S::b - 1) / S::b;
   static constexpr bool kDirRounds = NU == S::b;
-  // Blocks per SM of the register budget: three where a block is one cell
-  // (27^3 N=5 0.753 ms, with two 0.793, four 0.775); the 250- and 256-thread
-  // blocks of the lower orders spill there (25x21x19 N=4 0.232 ms with two,
-  // 0.263 with three).
-  static constexpr int BLOCKS = CPB == 1 && !PDE::kPointSource ? 3 : 2;  // (the point source's code needs more)
+  // Blocks per SM of the register budget: three where a block is one cell of
+  // N = 5 in 3D (27^3 0.753 ms, with two 0.793, four 0.775), else 512 threads
+  // (N=4 with five blocks of 125 threads 208 us, with four 206).
+  static constexpr int BLOCKS = S::P <= 128 ? 4 : PDE::kPointSource ? 2 : 3;  // (the point source's code needs more)
   static constexpr int NREG = regs_for_blocks<THREADS, BLOCKS>();
   static_assert(NU * DIM == NPAIRS, "as many components in every direction");
   static_assert(S::nD + NU >= 2 * S::nV, "the second direction's fluxes lie behind the first's");

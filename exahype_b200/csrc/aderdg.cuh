@@ -795,7 +795,13 @@ __device__ __forceinline__ double corrector_node(double* q, const double* __rest
 template <int DIM, int N, class PDE>
 struct CorrectorCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
-  static constexpr int CPB = cells_per_block<S::P>();
+  // What fits 128 threads, or one cell: the block is a chain of loads, one
+  // update and stores with barriers between them, and smaller blocks overlap
+  // better than ones of up to 256 threads (9,975 cells 3D N=4 elastic 109 ->
+  // 96 us, Euler 51 -> 48, 27^3 N=3 55 -> 46, 81^2 N=7 17 -> 15). Bound by
+  // memory: 27^3 N=5 140 us, 4.9 TB/s. No register budget: for 768 threads
+  // an SM the elastic one spills (133 us), at N=5 the loads are held back (171).
+  static constexpr int CPB = S::P <= 128 ? 128 / S::P : 1;
   // whole warps: the block min-reduction shuffles across full warps
   static constexpr int THREADS = (CPB * S::P + 31) / 32 * 32;
   // per cell in shared memory: state (node stride QS, odd against bank

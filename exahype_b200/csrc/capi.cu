@@ -180,6 +180,8 @@ struct KernelSet {
                   const int*, int, cudaStream_t);
   int (*plot)(const double*, double*, int, cudaStream_t);
   bool point_source;  // the PDE has a point source (usePointSource)
+  bool tmem;          // variants 0 and 8 are the tensor-memory form, which counts its sweeps itself
+  int predictor_launches(int variant) const { return linear || (tmem && (variant == 0 || variant == 8)) ? 1 : 2; }
 };
 
 template <int DIM, int N, class PDE>
@@ -397,6 +399,7 @@ struct Launch {
     using S = Shape<DIM, N, PDE>;
     KernelSet k{DIM, N, pde, S::nV, S::nP, S::P, S::F, false, &predictor, &riemann, &boundary, &corrector, nullptr};
     AmrLaunch<DIM, N, PDE>::fill(k);
+    k.tmem = kTmem;
     return k;
   }
 };
@@ -1539,7 +1542,7 @@ static int mesh_amr_faces(exa_mesh* m) {
 static int mesh_predict(exa_mesh* m, const int* count = nullptr, bool after_update = false) {
   const KernelSet& k = m->s->k;
   PhaseTimer pt(m, 0);
-  m->phase_launches[0] += 2;
+  m->phase_launches[0] += k.predictor_launches(m->s->variant);
   double* dt = m->fused ? (m->ref.on ? m->ref.lv + 2 * m->ref.nlev : m->scal + 5) : mesh_dt(m);
   Geometry g = m->geo;
   if (k.point_source) {

@@ -47,6 +47,30 @@ struct GradPairs {
   }
 };
 
+// Where the planes of a cell lie in shared memory: the nD of the state, then
+// the gradient components'. PL apart, except for six nodes in 3D with nine
+// variables: there a line's threads meet in few banks only if each plane's
+// position modulo the 16 banks of 64 bits is chosen by what is read and written
+// together. The residues come from a search over a count of the wavefronts of
+// the three directions' loads (state) and stores (components) with the item
+// orders of the kernel; 966 a level against 1188 with all planes PL apart
+// (882 if nothing met). The shared-memory pipe bounds the kernel (96 % busy
+// before): 27^3 N=5 757 -> 720 us.
+template <int PLANES, int PL, int CELL, bool PLACED>
+struct CKPlanes {
+  int at[PLANES + 1] = {};  // [PLANES]: the end
+  constexpr CKPlanes() {
+    constexpr int residue[30] = {0, 15, 1, 9, 5, 2, 11, 4, 13, 5, 14, 7,  // state (the last three are parameters)
+                                 0, 1, 2, 3, 4, 5,                       // components of x
+                                 0, 6, 12, 2, 8, 14,                     // y
+                                 0, 4, 8, 12, 0, 4};                     // z
+    for (int k = 1; k <= PLANES; k++) {
+      at[k] = at[k - 1] + (PLACED ? CELL : PL);
+      if (PLACED && k < PLANES) at[k] += (residue[k < 30 ? k : 0] - at[k] % 16 + 16) % 16;
+    }
+  }
+};
+
 template <int DIM, int N, class PDE>
 struct CKCfg : Shape<DIM, N, PDE> {
   using S = Shape<DIM, N, PDE>;
@@ -61,18 +85,20 @@ struct CKCfg : Shape<DIM, N, PDE> {
   // banks), plane pitch (odd: the variables of one node lie in different banks)
   static constexpr int YP = S::b == 4 ? 5 : S::b, ZP = S::b * YP;
   static constexpr int PL = (ZP * (DIM == 3 ? S::b : 1)) | 1;
-  static constexpr int SC = (S::nD + NPAIRS) * PL;  // doubles per cell
+  static constexpr bool kPlaced = DIM == 3 && S::b == 6 && S::nV == 9 && S::nD == 12 && NPAIRS == 18;
+  using Planes = CKPlanes<S::nD + NPAIRS, PL, S::b * ZP, kPlaced>;
+  static constexpr int SC = Planes().at[S::nD + NPAIRS];  // doubles per cell
   static constexpr size_t SMEM = sizeof(double) * (size_t)CPB * SC;
   // gradient items per thread; with NU == b one direction per round
   static constexpr int ROUNDS = (NPAIRS + S::b - 1) / S::b;
   static constexpr bool kDirRounds = NU == S::b;
   // Blocks per SM of the register budget: three where a block is one cell of
-  // N = 5 in 3D (27^3 0.753 ms, with two 0.793, four 0.775), else 512 threads
+  // N = 5 in 3D (27^3, planes PL apart: 0.753 ms, with two 0.793, four 0.775), else 512 threads
   // (N=4 with five blocks of 125 threads 208 us, with four 206).
   static constexpr int BLOCKS = S::P <= 128 ? 4 : PDE::kPointSource ? 2 : 3;  // (the point source's code needs more)
   static constexpr int NREG = regs_for_blocks<THREADS, BLOCKS>();
   static_assert(NU * DIM == NPAIRS, "as many components in every direction");
-  static_assert(S::nD + NU >= 2 * S::nV, "the second direction's fluxes lie behind the first's");
+  static_assert(Planes().at[S::nD + NU] >= 2 * S::nV * PL, "the second direction's fluxes lie behind the first's");
   static __host__ __device__ constexpr int pos(int x, int y, int z) { return z * ZP + y * YP + x; }
   static __host__ __device__ constexpr int step(int d) { return d == 0 ? 1 : d == 1 ? YP : ZP; }
   // first node of line L along d (L enumerates the other coordinates in
@@ -189,7 +215,15 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
   double* sC = smem + lc * C::SC;
   const int x = p % b, y = (p / b) % b, z = DIM == 3 ? p / (b * b) : 0;
   double* own = sC + C::pos(x, y, z);
-  double* ownG = own + nD * PL;
+  constexpr typename C::Planes PT;
+  __shared__ int s_plane[nD];  // the state's planes, for a variable known at run time
+  if constexpr (C::kPlaced) {
+#pragma unroll
+    for (int v = 0; v < nD; v++)
+      if (threadIdx.x == v) s_plane[v] = PT.at[v];
+    __syncthreads();
+  }
+  auto plane = [&](int v) { return C::kPlaced ? s_plane[v] : v * PL; };
   const int inst = cell_instance(geo, cell);
   const double dt = dt_ptr[inst];
   double idx[DIM];
@@ -219,13 +253,14 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     for (int k = 0; k < nD; k++) {
       const int e = p + k * P, n = e / nD, v = e - n * nD;
       const int nx = n % b, ny = (n / b) % b, nz = DIM == 3 ? n / (b * b) : 0;
-      sC[v * PL + C::pos(nx, ny, nz)] = active ? __ldg(src + e) : (v < nV ? 0.0 : 1.0);
+      sC[plane(v) + C::pos(nx, ny, nz)] = active ? __ldg(src + e) : (v < nV ? 0.0 : 1.0);
     }
   }
   // gradient items of this thread: component j of the pairs, line L.
   // Consecutive threads take consecutive lines of one component; along x
   // (with one direction per round) consecutive components of one line, whose
-  // lines start an even number of doubles apart.
+  // lines start an even number of doubles apart; along y, where the planes are
+  // placed for it, the lines of one z plane component by component.
   int g_src[C::ROUNDS], g_dst[C::ROUNDS];
 #pragma unroll
   for (int r = 0; r < C::ROUNDS; r++) {
@@ -233,6 +268,9 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     if (C::kDirRounds && r == 0) {
       L = p / NU;
       j = p % NU;
+    } else if (C::kPlaced && r == 1) {
+      L = p / (b * NU) * b + p % b;
+      j = p / b % NU + NU;
     } else {
       L = p % LINES;
       j = p / LINES + b * r;
@@ -241,13 +279,22 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     g_dst[r] = 0;
     if (j < C::NPAIRS) {
       constexpr GradPairs<PDE, DIM> GP;
-      int v = 0;
+      const int l0 = C::line0(j / NU, L);
+      if constexpr (C::kPlaced) {
 #pragma unroll
-      for (int i = 0; i < C::NPAIRS; i++)
-        if (i == j) v = GP.v[i];
-      const int d = j / NU, l0 = C::line0(d, L);
-      g_src[r] = v * PL + l0;
-      g_dst[r] = (nD + j) * PL + l0;
+        for (int i = 0; i < C::NPAIRS; i++)
+          if (i == j) {
+            g_src[r] = PT.at[GP.v[i]] + l0;
+            g_dst[r] = PT.at[nD + i] + l0;
+          }
+      } else {
+        int v = 0;
+#pragma unroll
+        for (int i = 0; i < C::NPAIRS; i++)
+          if (i == j) v = GP.v[i];
+        g_src[r] = v * PL + l0;
+        g_dst[r] = (nD + j) * PL + l0;
+      }
     }
   }
   auto gradients = [&]() {
@@ -275,15 +322,15 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     int i = 0;
 #pragma unroll
     for (int v = 0; v < nV; v++)
-      if (PDE::ncp_uses(d, v)) G[v] = idx[d] * ownG[(d * NU + i++) * PL];
+      if (PDE::ncp_uses(d, v)) G[v] = idx[d] * own[PT.at[nD + d * NU + i++]];
     PDE::ncp_dir(Qp, d, G, B);
   };
   __syncthreads();
   double Qp[nD], qh[nV];  // the node's parameters, the time-averaged state
 #pragma unroll
-  for (int v = 0; v < nV; v++) qh[v] = own[v * PL], Qp[v] = 0.0;
+  for (int v = 0; v < nV; v++) qh[v] = own[PT.at[v]], Qp[v] = 0.0;
 #pragma unroll
-  for (int v = nV; v < nD; v++) Qp[v] = own[v * PL];
+  for (int v = nV; v < nD; v++) Qp[v] = own[PT.at[v]];
   if constexpr (PS) {
     // a point source adds dt times its time integral to level 0
     // (3d/spaceTimePredictorLinear.cpph:77-90)
@@ -291,7 +338,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
       double psw[nV];
       node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
 #pragma unroll
-      for (int v = 0; v < nV; v++) own[v * PL] = qh[v] = __dadd_rn(qh[v], __dmul_rn(dt, psw[v]));
+      for (int v = 0; v < nV; v++) own[PT.at[v]] = qh[v] = __dadd_rn(qh[v], __dmul_rn(dt, psw[v]));
     }
     __syncthreads();
   }
@@ -317,7 +364,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
 #pragma unroll
     for (int v = 0; v < nV; v++) {
       qh[v] = fma(fac, qn[v], qh[v]);
-      own[v * PL] = last ? qh[v] : qn[v];
+      own[PT.at[v]] = last ? qh[v] : qn[v];
     }
     fac = fac * (dt / (i + 3));
   }
@@ -334,7 +381,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     for (int d = 0; d < DIM; d++)
       for (int it = p; it < LINES * nD; it += P) {
         const int L = it / nD, v = it - L * nD;
-        const double* q = sC + v * PL + C::line0(d, L);
+        const double* q = sC + plane(v) + C::line0(d, L);
         double sl = 0.0, sr = 0.0;
 #pragma unroll
         for (int l = 0; l < b; l++) {

@@ -46,10 +46,15 @@ __constant__ double c_amr_restr[3 * kAmrSq];
 __constant__ double c_amr_equi[kAmrSq];
 
 // A block works on one tensor of NAX axes with b nodes each and NV values per
-// node: one thread per line of the axis in turn (in ROUNDS rounds where a
-// block has fewer threads than lines). The lines of an axis are disjoint, so
-// every pass works in place in one shared buffer; the first pass reads its
-// lines from global memory and the last one writes its results there.
+// node: one thread per line of the axis in turn, in ROUNDS rounds where that is
+// more than 256 threads (order 7: 320). The 320 lines of 3D order 7 take one
+// round, the 432 of the elastic state at order 5 two, unrolled (but for sums into
+// global memory): in a loop over the rounds the compiler holds matrix entries in
+// registers across them and spills (transfers of order 7: 96 registers and up
+// to 884 bytes, now 50 and none; 5,832 of them: prolongation 77 -> 54 us,
+// restriction 76 -> 56, vertex projection 71 -> 68). The lines of an axis are
+// disjoint, so every pass works in place in one shared buffer; the first pass
+// reads its lines from global memory and the last one writes its results there.
 // Consecutive threads take consecutive values of the x rows, so the last
 // axis (of two or three) is written coalesced; the first (x) pass reads each row
 // whole, through L1. In the buffer the x rows (b NV values) have a pitch of
@@ -58,7 +63,7 @@ __constant__ double c_amr_equi[kAmrSq];
 template <int b, int NAX, int NV>
 struct TensorCfg {
   static constexpr int LINES = NV * ipow(b, NAX - 1), SIZE = LINES * b;
-  static constexpr int ROUNDS = (LINES + 255) / 256;
+  static constexpr int ROUNDS = b >= 8 ? (LINES + 319) / 320 : (LINES + 255) / 256;
   static constexpr int THREADS = ((LINES + ROUNDS - 1) / ROUNDS + 31) / 32 * 32;
   static constexpr int ROW = b * NV, ROWS = ipow(b, NAX - 1);
   static constexpr int PITCH = ROW + ((NV - ROW) % 16 + 16) % 16;
@@ -81,10 +86,10 @@ enum class Place { kBuffer, kGlobal, kGlobalAdd };
 // out[.., m, ..] = sum_n M[m][n] in[.., n, ..] along axis AX, M given as a
 // constant-memory pointer and row / column strides (compile-time indices: the
 // coefficients are constant-bank operands). `tid` of `THREADS` threads.
-template <class C, int b, int AX, int RS, int CS, Place FROM, Place TO, bool ROLLED = false>
+template <class C, int b, int AX, int RS, int CS, Place FROM, Place TO>
 __device__ __forceinline__ void apply_axis(const double* src, double* dst, double* buf, const double* M, int tid) {
   constexpr int ROW = C::ROW;
-#pragma unroll 1
+#pragma unroll(TO == Place::kGlobalAdd ? 1 : C::ROUNDS)
   for (int r = 0; r < C::ROUNDS; r++) {
     const int it = tid + r * C::THREADS;
     if (it >= C::LINES) break;
@@ -97,7 +102,7 @@ __device__ __forceinline__ void apply_axis(const double* src, double* dst, doubl
     double x[b];
 #pragma unroll
     for (int n = 0; n < b; n++) x[n] = FROM == Place::kBuffer ? in[n * is] : __ldg(in + n * is);
-#pragma unroll(ROLLED ? 1 : b)
+#pragma unroll
     for (int m = 0; m < b; m++) {
       double s = 0.0;
 #pragma unroll
@@ -110,19 +115,14 @@ __device__ __forceinline__ void apply_axis(const double* src, double* dst, doubl
   }
 }
 
-// one axis of a single-level transfer: the digit picks the third; each case
+// one axis of one level: the digit picks the third; each case
 // has a compile-time table address, so that the coefficients are constant-bank
-// operands (prolongation P[n][m], restriction R[m][n]). DEEP (a level among
-// several, in a loop): one form for the three thirds, its coefficients loaded
-// where they are used -- the compiler would hold all matrices in registers
-// across that loop.
-template <class C, int N, int AX, bool R, Place FROM, Place TO, bool DEEP>
+// operands (prolongation P[n][m], restriction R[m][n])
+template <class C, int N, int AX, bool R, Place FROM, Place TO>
 __device__ __forceinline__ void transfer_axis(const double* src, double* dst, double* buf, int digit, int tid) {
   constexpr int b = N + 1, base = 3 * amr_off(N), RS = R ? b : 1, CS = R ? 1 : b;
   const double* tab = R ? c_amr_restr : c_amr_fine;
-  if constexpr (DEEP)
-    apply_axis<C, b, AX, RS, CS, FROM, TO, true>(src, dst, buf, tab + base + digit * b * b, tid);
-  else if (digit == 0) {
+  if (digit == 0) {
     apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base, tid);
   } else if (digit == 1) {
     apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base + b * b, tid);
@@ -142,18 +142,30 @@ __device__ __forceinline__ void part_sync() {
 }
 
 // the axes of one level in turn
-template <int N, int NAX, int NV, bool R, Place FROM, Place TO, int ID, bool DEEP = false>
+template <int N, int NAX, int NV, bool R, Place FROM, Place TO, int ID>
 __device__ __forceinline__ void transfer_level(const double* src, double* dst, double* buf, const int* digit, int tid) {
   using C = TensorCfg<N + 1, NAX, NV>;
-  transfer_axis<C, N, 0, R, FROM, NAX == 1 ? TO : Place::kBuffer, DEEP>(src, dst, buf, digit[0], tid);
+  transfer_axis<C, N, 0, R, FROM, NAX == 1 ? TO : Place::kBuffer>(src, dst, buf, digit[0], tid);
   if constexpr (NAX > 1) {
     part_sync<ID, C::THREADS>();
-    transfer_axis<C, N, 1, R, Place::kBuffer, NAX == 2 ? TO : Place::kBuffer, DEEP>(src, dst, buf, digit[1], tid);
+    transfer_axis<C, N, 1, R, Place::kBuffer, NAX == 2 ? TO : Place::kBuffer>(src, dst, buf, digit[1], tid);
   }
   if constexpr (NAX > 2) {
     part_sync<ID, C::THREADS>();
-    transfer_axis<C, N, 2, R, Place::kBuffer, TO, DEEP>(src, dst, buf, digit[2], tid);
+    transfer_axis<C, N, 2, R, Place::kBuffer, TO>(src, dst, buf, digit[2], tid);
   }
+}
+
+// The same as a function of its own, for the loop over several levels: inlined
+// there, the compiler loads the matrices of all thirds into registers before
+// the loop (spills of up to 2 KB); with one rolled form for the three thirds
+// every coefficient is a load of its own (19,683 transfers of 3D N=5 over two
+// levels 203 us, so 101). buf: shared-memory address.
+template <int N, int NAX, int NV, bool R, Place FROM, Place TO, int ID>
+__device__ __noinline__ void transfer_level_call(const double* src, double* dst, uint32_t buf, int d0, int d1, int d2,
+                                                 int tid) {
+  const int digit[3] = {d0, d1, d2};
+  transfer_level<N, NAX, NV, R, FROM, TO, ID>(src, dst, (double*)__cvta_shared_to_generic(buf), digit, tid);
 }
 
 // levelDelta in 1..kMaxLevelDelta and every index digit-string in
@@ -180,6 +192,7 @@ __device__ __forceinline__ void amr_transfer(const double* __restrict__ src, dou
     transfer_level<N, NAX, NV, R, Place::kGlobal, TO, ID>(src, dst, buf, index, tid);
     return;
   }
+  const uint32_t sbuf = (uint32_t)__cvta_generic_to_shared(buf);
   int rest[3] = {index[0], index[1], index[2]};
   int sig = 1;
   for (int l = 1; l < levelDelta; l++) sig *= 3;
@@ -198,12 +211,13 @@ __device__ __forceinline__ void amr_transfer(const double* __restrict__ src, dou
     }
     sig = sig > 1 ? sig / 3 : 1;
     if (l > 0) part_sync<ID, TensorCfg<N + 1, NAX, NV>::THREADS>();
+    const int d0 = digit[0], d1 = digit[1], d2 = digit[2];
     if (l == 0)
-      transfer_level<N, NAX, NV, R, Place::kGlobal, Place::kBuffer, ID, true>(src, dst, buf, digit, tid);
+      transfer_level_call<N, NAX, NV, R, Place::kGlobal, Place::kBuffer, ID>(src, dst, sbuf, d0, d1, d2, tid);
     else if (l + 1 < levelDelta)
-      transfer_level<N, NAX, NV, R, Place::kBuffer, Place::kBuffer, ID, true>(src, dst, buf, digit, tid);
+      transfer_level_call<N, NAX, NV, R, Place::kBuffer, Place::kBuffer, ID>(src, dst, sbuf, d0, d1, d2, tid);
     else
-      transfer_level<N, NAX, NV, R, Place::kBuffer, TO, ID, true>(src, dst, buf, digit, tid);
+      transfer_level_call<N, NAX, NV, R, Place::kBuffer, TO, ID>(src, dst, sbuf, d0, d1, d2, tid);
   }
 }
 

@@ -1,6 +1,6 @@
-"""AMR transfers and the vertex projection at the shapes where an axis has more
-lines than a block has threads (order 7: 320 lines; the elastic state at order
-5: 432) and at 2D order 7, with the checks and the bound of test_gpu_amr
+"""AMR transfers and the vertex projection at the shapes around the line where an
+axis has more lines than a block has threads (3D order 7: 320 lines, one round;
+the elastic state at order 5: 432, two) and at 2D order 7, with the checks and the bound of test_gpu_amr
 (1e-12 of the largest value: the same sums in another order)."""
 import pytest
 

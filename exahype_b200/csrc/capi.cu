@@ -2363,7 +2363,9 @@ struct LimLaunch {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PROJ_SMEM * PC::CELLS)));
     EXA_CUDA(cudaFuncSetAttribute(lim_recompute_kernel<DIM, N, PDE, typename PC::Group>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PROJ_SMEM * PC::CELLS)));
-    EXA_CUDA(cudaFuncSetAttribute(lim_project_kernel<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    EXA_CUDA(cudaFuncSetAttribute(lim_project_kernel<DIM, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)PROJ_SMEM));
+    EXA_CUDA(cudaFuncSetAttribute(lim_project_kernel<DIM, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)PROJ_SMEM));
     done = true;
     return EXA_OK;
@@ -2410,7 +2412,10 @@ struct LimLaunch {
     if (n <= 0) return EXA_OK;
     int rc = attrs();
     if (rc) return rc;
-    lim_project_kernel<DIM, N><<<n, 128, PROJ_SMEM, st>>>(list, n, luh, lim, to_fv);
+    if (to_fv)
+      lim_project_kernel<DIM, N, true><<<n, 128, PROJ_SMEM, st>>>(list, n, luh, lim);
+    else
+      lim_project_kernel<DIM, N, false><<<n, 128, PROJ_SMEM, st>>>(list, n, luh, lim);
     EXA_LAUNCHED();
     return EXA_OK;
   }

@@ -1298,19 +1298,26 @@ __global__ void __launch_bounds__(128) lim_recompute_kernel(int ncells, double* 
 }
 
 // Batched projections for the kernel-level entry points: one block per listed
-// cell (list NULL: cells 0..n-1). to_fv: luh -> interior subcells of lim,
-// else interior subcells of lim -> luh.
-template <int DIM, int N>
-__global__ void __launch_bounds__(128) lim_project_kernel(const int* __restrict__ list, int n,
-                                                          double* __restrict__ luh, double* __restrict__ lim,
-                                                          int to_fv) {
+// cell (list NULL: cells 0..n-1). TO_FV: luh -> interior subcells of lim, else
+// interior subcells of lim -> luh. One kernel per direction, each with its own
+// register budget (blocks per SM, 0: none stated): with both in one kernel the
+// compiler held matrix entries of the way to the DG basis in registers (124 at
+// order 7; 20,000 patches 2D N=7 191 us, with eight blocks 70, none stated 89;
+// 3,000 patches 3D N=7 606, with one stated 400; N=5 66, 58, none stated 72). To
+// the subcells any stated number costs (3,000 cells 3D N=7 212 us, with one 257,
+// four 232).
+template <int DIM, bool TO_FV>
+constexpr int project_blocks() { return TO_FV ? 0 : DIM == 2 ? 8 : 1; }
+template <int DIM, int N, bool TO_FV>
+__global__ void __launch_bounds__(128, project_blocks<DIM, TO_FV>())
+    lim_project_kernel(const int* __restrict__ list, int n, double* __restrict__ luh, double* __restrict__ lim) {
   using L = LimShape<DIM, N>;
   extern __shared__ double tmp[];
   if ((int)blockIdx.x >= n) return;
   const int c = list ? list[blockIdx.x] : (int)blockIdx.x;
   double* u = luh + (size_t)c * L::P * L::nV;
   double* l = lim + (size_t)c * L::LS;
-  if (to_fv)
+  if constexpr (TO_FV)
     project_fv_block<DIM, N>(u, l, tmp);
   else
     project_dg_block<DIM, N>(l, u, tmp);

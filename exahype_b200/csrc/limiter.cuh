@@ -429,9 +429,11 @@ struct MusclCfg {
   // phases, so what counts is how many are in flight: three blocks an SM up to
   // N = 5 (81^2 N=5, about a tenth of the cells: 20.5 us with 256 threads and
   // the neighbours read from global memory, 16.2 with two blocks, 13.5 with
-  // three); N = 7 spills at two (25^2, 40 limiting steps 4.75 ms, with one 4.50).
-  static constexpr int THREADS = (2 * NE + 31) / 32 * 32;
-  static constexpr int MINB = THREADS <= 320 ? 3 : 1;
+  // three). At N = 7 shared memory holds two blocks; for their registers the 480
+  // edges take two rounds of 320 threads (one block of 480 threads is as fast up to
+  // 148 patches, 11 us; 300: 25 -> 21, 1,000: 58 -> 42, 4,000: 241 -> 158).
+  static constexpr int THREADS = N == 7 ? 320 : (2 * NE + 31) / 32 * 32;
+  static constexpr int MINB = N == 7 ? 2 : 3;
   static constexpr size_t SMEM = sizeof(double) * (U + W + FX);
   static_assert(NR <= THREADS, "one subcell of the ring per thread");
   static_assert(tensor_tmp<2, L::B, L::b>() <= W, "the projection's scratch takes the states' place");
@@ -539,8 +541,9 @@ __global__ void __launch_bounds__(MusclCfg<N>::THREADS, MusclCfg<N>::MINB)
     __syncthreads();
     // Rusanov flux on every subcell edge: edge e of direction d
     // joins positions k and k+1 along d, k in [-1, B) relative to the interior
-    if (threadIdx.x < DIM * C::NE) {
-      const int i = threadIdx.x, d = i / C::NE, e = i % C::NE;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < DIM * C::NE; i += C::THREADS) {
+      const int d = i / C::NE, e = i % C::NE;
       const int kk = e % (B + 1), t = e / (B + 1);  // position k + 1 along d, transverse interior coordinate
       const int qL = d == 0 ? (t + 1) * R + kk : kk * R + t + 1;  // ring index 0 = first ghost layer
       const int qR = qL + (d == 0 ? 1 : R);

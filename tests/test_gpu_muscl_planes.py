@@ -12,6 +12,11 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
+def test_muscl_2d_edges_in_two_rounds(eb):  # noqa: F811
+    """2D order 7, where a block has fewer threads than a patch has edges"""
+    lk.test_musclhancock_update_vs_oracle(eb, 2, 7, 19)
+
+
 @pytest.mark.parametrize("order,n", [(4, 5), (7, 2)])
 def test_muscl_planes_vs_oracle(eb, order, n):  # noqa: F811
     lk.test_musclhancock_update_vs_oracle(eb, 3, order, n)

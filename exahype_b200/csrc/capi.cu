@@ -21,6 +21,7 @@
 #include "limiter.cuh"
 #include "linear.cuh"
 #include "amr.cuh"
+#include "device_once.h"
 
 namespace exa {
 
@@ -238,12 +239,8 @@ static int launch_corrector(double* luh, const double* du, const double* fb, con
                             Geometry g, int n, const int* list, int upd, const int* cnt, cudaStream_t st) {
   using CC = CorrectorCfg<DIM, N, PDE>;
   if (n <= 0) return EXA_OK;
-  static bool attr = false;
-  if (!attr) {
-    EXA_CUDA(cudaFuncSetAttribute(corrector_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)CC::SMEM));
-    attr = true;
-  }
+  static DeviceOnce once;
+  EXA_CUDA(once([] { return allow_smem(corrector_kernel<DIM, N, PDE>, CC::SMEM); }));
   corrector_kernel<DIM, N, PDE><<<(n + CC::CPB - 1) / CC::CPB, CC::THREADS, CC::SMEM, st>>>(luh, du, fb, dt, dtout, g,
                                                                                            n, list, upd, cnt);
   EXA_LAUNCHED();
@@ -275,12 +272,8 @@ struct Launch {
   static int launch_pred(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
                          Geometry g, int n, const int* list, const int* cnt, PredictorTemps tmp, cudaStream_t st) {
     using PC = PredictorCfg<DIM, N, PDE, VS, MB>;
-    static bool attr = false;
-    if (!attr) {
-      EXA_CUDA(cudaFuncSetAttribute(predictor_kernel<DIM, N, PDE, TEMPS, VS, MB>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC::SMEM));
-      attr = true;
-    }
+    static DeviceOnce once;
+    EXA_CUDA(once([] { return allow_smem(predictor_kernel<DIM, N, PDE, TEMPS, VS, MB>, PC::SMEM); }));
     const int grid = (n + PC::CPB - 1) / PC::CPB;
     predictor_kernel<DIM, N, PDE, TEMPS, VS, MB><<<grid, PC::THREADS, PC::SMEM, st>>>(luh, qb, fb, du, iters, dt, g,
                                                                                      n, list, tmp, cnt);
@@ -292,12 +285,8 @@ struct Launch {
   static int launch_lines(const double* luh, double* qb, double* fb, double* du, int* iters, const double* dt,
                           Geometry g, int n, const int* list, const int* cnt, PredictorTemps tmp, cudaStream_t st) {
     using LC = LinesCfg<DIM, N, PDE, MB, MIXED, TS>;
-    static bool attr = false;
-    if (!attr) {
-      EXA_CUDA(cudaFuncSetAttribute(predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LC::SMEM));
-      attr = true;
-    }
+    static DeviceOnce once;
+    EXA_CUDA(once([] { return allow_smem(predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS>, LC::SMEM); }));
     const int grid = (n + LC::CPB - 1) / LC::CPB;
     predictor_lines_kernel<DIM, N, PDE, TEMPS, MB, MIXED, TS>
         <<<grid, LC::THREADS, LC::SMEM, st>>>(luh, qb, fb, du, iters, dt, g, n, list, tmp, cnt);
@@ -322,12 +311,8 @@ struct Launch {
                          cudaStream_t st) {
     if constexpr (kTmem) {
       using TC = TmemCfg<DIM, N, PDE, FEW>;
-      static bool attr = false;
-      if (!attr) {
-        EXA_CUDA(cudaFuncSetAttribute(predictor_tmem_kernel<DIM, N, PDE, FEW>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC::SMEM));
-        attr = true;
-      }
+      static DeviceOnce once;
+      EXA_CUDA(once([] { return allow_smem(predictor_tmem_kernel<DIM, N, PDE, FEW>, TC::SMEM); }));
       predictor_tmem_kernel<DIM, N, PDE, FEW><<<(n + TC::CPB - 1) / TC::CPB, TC::THREADS, TC::SMEM, st>>>(
           luh, qb, fb, du, iters, acc, dt, g, n, list, cnt);
       EXA_LAUNCHED();
@@ -418,12 +403,8 @@ struct LinearLaunch {
                        int n, const int* list, const int* cnt, PredictorTemps tmp, bool temps, unsigned long long*,
                        int, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    static bool attr = false;
-    if (!attr) {
-      EXA_CUDA(cudaFuncSetAttribute(ck_predictor_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)KC::SMEM));
-      attr = true;
-    }
+    static DeviceOnce once;
+    EXA_CUDA(once([] { return allow_smem(ck_predictor_kernel<DIM, N, PDE>, KC::SMEM); }));
     ck_predictor_kernel<DIM, N, PDE><<<(n + KC::CPB - 1) / KC::CPB, KC::THREADS, KC::SMEM, st>>>(
         luh, qb, fb, du, dt, g, n, list, cnt, temps ? tmp.lQhi : nullptr, temps ? tmp.lFhi : nullptr);
     EXA_LAUNCHED();
@@ -2349,30 +2330,32 @@ struct LimLaunch {
   static constexpr size_t PROJ_SMEM = sizeof(double) * PROJ_TMP;
   static_assert(MC::SMEM <= 227 * 1024 && PC::SMEM <= 227 * 1024 && PROJ_SMEM <= 227 * 1024, "shared memory");
 
+  // the shared-memory limits of the kernels below, but for the patch update's
   static int attrs() {
-    static bool done = false;
-    if (done) return EXA_OK;
+    static DeviceOnce once;
+    EXA_CUDA(once([] {
+      using G = typename PC::Group;
+      const cudaError_t r[] = {allow_smem(lim_post_update_kernel<DIM, N, PDE, G>, PC::POST_SMEM),
+                               allow_smem(lim_init_kernel<DIM, N, PDE>, PC::SMEM),
+                               allow_smem(lim_seed_kernel<DIM, N>, PROJ_SMEM),
+                               allow_smem(lim_reinit_kernel<DIM, N, G>, PROJ_SMEM * PC::CELLS),
+                               allow_smem(lim_recompute_kernel<DIM, N, PDE, G>, PROJ_SMEM * PC::CELLS),
+                               allow_smem(lim_project_kernel<DIM, N, true>, PROJ_SMEM),
+                               allow_smem(lim_project_kernel<DIM, N, false>, PROJ_SMEM)};
+      for (const cudaError_t e : r)
+        if (e != cudaSuccess) return e;
+      return cudaSuccess;
+    }));
+    return EXA_OK;
+  }
+  // set on every call of the kernel-level entry point, at mesh creation for the step
+  static int muscl_attr() {
     EXA_CUDA(cudaFuncSetAttribute(muscl_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MC::SMEM));
-    EXA_CUDA(cudaFuncSetAttribute(lim_post_update_kernel<DIM, N, PDE, typename PC::Group>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PC::POST_SMEM));
-    EXA_CUDA(cudaFuncSetAttribute(lim_init_kernel<DIM, N, PDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PC::SMEM));
-    EXA_CUDA(cudaFuncSetAttribute(lim_seed_kernel<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PROJ_SMEM));
-    EXA_CUDA(cudaFuncSetAttribute(lim_reinit_kernel<DIM, N, typename PC::Group>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PROJ_SMEM * PC::CELLS)));
-    EXA_CUDA(cudaFuncSetAttribute(lim_recompute_kernel<DIM, N, PDE, typename PC::Group>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PROJ_SMEM * PC::CELLS)));
-    EXA_CUDA(cudaFuncSetAttribute(lim_project_kernel<DIM, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PROJ_SMEM));
-    EXA_CUDA(cudaFuncSetAttribute(lim_project_kernel<DIM, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PROJ_SMEM));
-    done = true;
     return EXA_OK;
   }
   // MUSCL blocks resident on the device at once (grid-stride over the FV list)
   static int muscl_grid(int ncells, int* grid) {
-    EXA_CUDA(cudaFuncSetAttribute(muscl_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MC::SMEM));
+    if (const int rc = muscl_attr()) return rc;
     int dev = 0, sms = 0, per_sm = 0;
     EXA_CUDA(cudaGetDevice(&dev));
     EXA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2386,7 +2369,7 @@ struct LimLaunch {
                         const int* list, const double* scratch, size_t scratch_doubles_avail, bool needs_scratch,
                         cudaStream_t st) {
     if (n <= 0) return EXA_OK;
-    int rc = attrs();
+    int rc = muscl_attr();
     if (rc) return rc;
     if constexpr (kShare > 0)
       if (needs_scratch && (!scratch || scratch_doubles_avail < kShare))

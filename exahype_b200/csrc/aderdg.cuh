@@ -514,8 +514,9 @@ constexpr int scatter_lane(int k) {
 }
 
 // The quadrature averages of both sides of a face (QL, QR staged in shared
-// memory, FaceStage), spread over the warp: lanes 0..15 end with the left side's average, lanes
-// 16..31 with the right side's.
+// memory, FaceStage), spread over the warp: lanes 0..15 end with the left side's
+// average, lanes 16..31 with the right side's. With more than 16 values per node
+// (both sides' are more than a warp has lanes) every value is summed over all lanes.
 template <int DIM, int N, class PDE>
 struct FaceStage : Shape<DIM, N, PDE> {  // a face's states in shared memory
   using S = Shape<DIM, N, PDE>;
@@ -530,7 +531,6 @@ __device__ __forceinline__ void face_averages(const double* QL, const double* QR
   using S = Shape<DIM, N, PDE>;
   const OrderTables& T = c_tab[N];
   constexpr int M = 2 * S::nD;
-  static_assert(M <= 32, "one value per lane at the end");
   double a[M];
 #pragma unroll
   for (int k = 0; k < M; k++) a[k] = 0.0;
@@ -542,10 +542,19 @@ __device__ __forceinline__ void face_averages(const double* QL, const double* QR
       a[S::nD + k] += wf * QR[fn * FaceStage<DIM, N, PDE>::PITCH + k];
     }
   }
-  warp_sum_scatter<M>(a, lane);
+  if constexpr (M <= 32) {
+    warp_sum_scatter<M>(a, lane);
 #pragma unroll
-  for (int k = 0; k < S::nD; k++)
-    avg[k] = __shfl_sync(0xffffffffu, a[0], (lane & 16) | scatter_lane<M>(k));
+    for (int k = 0; k < S::nD; k++)
+      avg[k] = __shfl_sync(0xffffffffu, a[0], (lane & 16) | scatter_lane<M>(k));
+  } else {
+#pragma unroll
+    for (int k = 0; k < M; k++)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+#pragma unroll
+    for (int k = 0; k < S::nD; k++) avg[k] = lane < 16 ? a[k] : a[S::nD + k];
+  }
 }
 
 // max_v |lambda_v| of one state

@@ -32,18 +32,26 @@
 
 namespace exa {
 
-// the (direction, variable) gradient components the PDE's ncp reads
+// the (direction, variable) gradient components the PDE's ncp reads, direction
+// by direction; those of direction e are first[e] .. first[e + 1] - 1
 template <class PDE, int DIM>
 struct GradPairs {
-  int d[DIM * PDE::nVar], v[DIM * PDE::nVar], n;
-  constexpr GradPairs() : d(), v(), n(0) {
-    for (int dd = 0; dd < DIM; dd++)
+  int d[DIM * PDE::nVar], v[DIM * PDE::nVar], first[DIM + 1], n;
+  constexpr GradPairs() : d(), v(), first(), n(0) {
+    for (int dd = 0; dd < DIM; dd++) {
       for (int vv = 0; vv < PDE::nVar; vv++)
         if (PDE::ncp_uses(dd, vv)) {
           d[n] = dd;
           v[n] = vv;
           n++;
         }
+      first[dd + 1] = n;
+    }
+  }
+  constexpr bool even() const {  // as many in every direction
+    for (int dd = 0; dd < DIM; dd++)
+      if ((first[dd + 1] - first[dd]) * DIM != n) return false;
+    return true;
   }
 };
 
@@ -80,12 +88,14 @@ struct CKCfg : Shape<DIM, N, PDE> {
   static constexpr int CPB = S::P <= 128 ? 128 / S::P : 1;
   static constexpr int THREADS = CPB * S::P;
   static constexpr int LINES = S::F;                                             // lines per direction
-  static constexpr int NPAIRS = GradPairs<PDE, DIM>().n, NU = NPAIRS / DIM;  // gradient components, per direction
+  static constexpr int NPAIRS = GradPairs<PDE, DIM>().n;  // gradient components
+  static constexpr bool kEven = GradPairs<PDE, DIM>().even();
+  static constexpr int NU = kEven ? NPAIRS / DIM : 1;  // per direction, where as many in each (b > 1)
   // planes: row pitch (4 nodes: 5, or the x lines' threads would meet in four
   // banks), plane pitch (odd: the variables of one node lie in different banks)
   static constexpr int YP = S::b == 4 ? 5 : S::b, ZP = S::b * YP;
   static constexpr int PL = (ZP * (DIM == 3 ? S::b : 1)) | 1;
-  static constexpr bool kPlaced = DIM == 3 && S::b == 6 && S::nV == 9 && S::nD == 12 && NPAIRS == 18;
+  static constexpr bool kPlaced = kEven && DIM == 3 && S::b == 6 && S::nV == 9 && S::nD == 12 && NPAIRS == 18;
   using Planes = CKPlanes<S::nD + NPAIRS, PL, S::b * ZP, kPlaced>;
   static constexpr int SC = Planes().at[S::nD + NPAIRS];  // doubles per cell
   static constexpr size_t SMEM = sizeof(double) * (size_t)CPB * SC;
@@ -97,8 +107,11 @@ struct CKCfg : Shape<DIM, N, PDE> {
   // (N=4 with five blocks of 125 threads 208 us, with four 206).
   static constexpr int BLOCKS = S::P <= 128 ? 4 : PDE::kPointSource ? 2 : 3;  // (the point source's code needs more)
   static constexpr int NREG = regs_for_blocks<THREADS, BLOCKS>();
-  static_assert(NU * DIM == NPAIRS, "as many components in every direction");
-  static_assert(Planes().at[S::nD + NU] >= 2 * S::nV * PL, "the second direction's fluxes lie behind the first's");
+  // the second direction's fluxes lie behind the first's where the planes up to
+  // its gradient components hold both (few components or no parameters: in the
+  // first's place, after one more barrier)
+  static constexpr bool kBehind = Planes().at[S::nD + GradPairs<PDE, DIM>().first[1]] >= 2 * S::nV * PL;
+  static_assert(Planes().at[S::nD] >= S::nV * PL, "the first direction's fluxes take the place of the state");
   static __host__ __device__ constexpr int pos(int x, int y, int z) { return z * ZP + y * YP + x; }
   static __host__ __device__ constexpr int step(int d) { return d == 0 ? 1 : d == 1 ? YP : ZP; }
   // first node of line L along d (L enumerates the other coordinates in
@@ -279,7 +292,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     g_dst[r] = 0;
     if (j < C::NPAIRS) {
       constexpr GradPairs<PDE, DIM> GP;
-      const int l0 = C::line0(j / NU, L);
+      const int l0 = C::line0(j < GP.first[1] ? 0 : DIM == 2 || j < GP.first[2] ? 1 : 2, L);
       if constexpr (C::kPlaced) {
 #pragma unroll
         for (int i = 0; i < C::NPAIRS; i++)
@@ -304,8 +317,9 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
       int st;
       if (C::kDirRounds) st = C::step(r);
       else {
-        const int d = (g_dst[r] / PL - nD) / NU;
-        st = d == 0 ? C::step(0) : d == 1 ? C::step(1) : C::step(2);
+        constexpr GradPairs<PDE, DIM> GP;
+        const int j = g_dst[r] / PL - nD;
+        st = j < GP.first[1] ? C::step(0) : DIM == 2 || j < GP.first[2] ? C::step(1) : C::step(2);
       }
       const double* s = sC + g_src[r];
       double* g = sC + g_dst[r];
@@ -322,7 +336,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     int i = 0;
 #pragma unroll
     for (int v = 0; v < nV; v++)
-      if (PDE::ncp_uses(d, v)) G[v] = idx[d] * own[PT.at[nD + d * NU + i++]];
+      if (PDE::ncp_uses(d, v)) G[v] = idx[d] * own[PT.at[nD + GradPairs<PDE, DIM>().first[d] + i++]];
     PDE::ncp_dir(Qp, d, G, B);
   };
   __syncthreads();
@@ -395,8 +409,8 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
   }
   __syncthreads();
   // time-averaged fluxes one direction at a time: the node's values to shared
-  // memory (where nothing is read any more: the state planes, then the planes
-  // behind the first direction's fluxes, then the first's again), their
+  // memory (where nothing is read any more: the state planes, then, where they fit,
+  // the planes behind the first direction's fluxes, then the first's again), their
   // extrapolation from there; volumeIntegralLinear is pointwise
   double du[nV];
   double psw[nV];
@@ -414,11 +428,13 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
 #pragma unroll
         for (int v = 0; v < nV; v++) B[v] = __dadd_rn(B[v], __ddiv_rn(psw[v], (double)DIM));
     }
-    double* st = sC + (d == 1 ? nV * PL : 0);
+    constexpr int BEHIND = C::kBehind ? nV * PL : 0;
+    if (!C::kBehind && d > 0) __syncthreads();
+    double* st = sC + (d == 1 ? BEHIND : 0);
 #pragma unroll
     for (int v = 0; v < nV; v++) {
       du[v] -= w * B[v];
-      (own + (d == 1 ? nV * PL : 0))[v * PL] = B[v];
+      (own + (d == 1 ? BEHIND : 0))[v * PL] = B[v];
     }
     if (lFhi_out && active)
 #pragma unroll

@@ -227,15 +227,18 @@ struct EulerSourceNCPPDE : EulerTestPDE {
 // 31-235): variables sxx syy szz sxy syz sxz u v w, material parameters
 // lambda mu rho. A linear PDE supplies what the reference's linear kernels
 // ask of the user solver instead of a flux:
-//   ncp<DIM>(Q, gradQ[DIM][nVar], BgradQ[DIM][nVar]) -- nonConservativeProduct
-//                                                       (BgradQ a DIM x nVar tensor)
-//   ncp_dir(Q, d, gradQ_d, BgradQ_d)                  -- its direction-d part
-//   coefficient_matrix(Q, d, Bn[nVar][nVar])          -- coefficientMatrix
-//   eigenvalues(Q, d, lambda)                         -- eigenvalues
-// with (BgradQ_d)_k = sum_l Bn_d[l][k] (gradQ_d)_l, and
-//   ncp_uses(d, v)  which gradient components ncp reads (no counterpart in
-//                   the reference, which computes them all). The z-direction parts are
-// the ones written out (commented) beside the x and y parts in the test.
+//   ncp_dir(Q, d, gradQ_d, BgradQ_d)  -- the direction-d part of
+//                                        nonConservativeProduct; applied to a
+//                                        jump it is the product with
+//                                        coefficientMatrix that the Riemann
+//                                        solver needs:
+//                                        (BgradQ_d)_k = sum_l Bn_d[l][k] (gradQ_d)_l
+//   eigenvalues(Q, d, lambda)         -- eigenvalues
+//   ncp_uses(d, v)  which gradient components ncp_dir reads (any number per
+//                   direction; no counterpart in the reference, which computes
+//                   them all)
+// The z-direction parts are the ones written out (commented) beside the x and y
+// parts in the test.
 struct ElasticPDE {
   static constexpr int nVar = 9;
   static constexpr int nPar = 3;
@@ -295,35 +298,12 @@ struct ElasticPDE {
     }
   }
 
-  template <int DIM>
-  __device__ static void ncp(const double* Q, const double (*G)[nVar], double (*B)[nVar]) {
-#pragma unroll
-    for (int d = 0; d < DIM; d++) ncp_dir(Q, d, G[d], B[d]);
-  }
-
-  // which gradient components ncp reads: direction d, variable v (the
+  // which gradient components ncp_dir reads: direction d, variable v (the
   // predictor computes only these; the others would not change its result)
   __host__ __device__ static constexpr bool ncp_uses(int d, int v) {
     return d == 0 ? (v == 0 || v == 3 || v == 5 || v >= 6)
          : d == 1 ? (v == 1 || v == 3 || v == 4 || v >= 6)
                   : (v == 2 || v == 4 || v == 5 || v >= 6);
-  }
-
-  // Bn row-major [l][k], all other entries zero
-  __device__ static void coefficient_matrix(const double* Q, int d, double* Bn) {
-    for (int i = 0; i < nVar * nVar; i++) Bn[i] = 0.0;
-    const double lam = Q[9], mu = Q[10], irho = 1.0 / Q[11];
-    const double lm2 = lam + 2 * mu;
-    if (d == 0) {
-      Bn[6 * 9 + 0] = -lm2; Bn[6 * 9 + 1] = -lam; Bn[6 * 9 + 2] = -lam; Bn[7 * 9 + 3] = -mu; Bn[8 * 9 + 5] = -mu;
-      Bn[0 * 9 + 6] = -irho; Bn[3 * 9 + 7] = -irho; Bn[5 * 9 + 8] = -irho;
-    } else if (d == 1) {
-      Bn[7 * 9 + 0] = -lam; Bn[7 * 9 + 1] = -lm2; Bn[7 * 9 + 2] = -lam; Bn[6 * 9 + 3] = -mu; Bn[8 * 9 + 4] = -mu;
-      Bn[3 * 9 + 6] = -irho; Bn[1 * 9 + 7] = -irho; Bn[4 * 9 + 8] = -irho;
-    } else {
-      Bn[8 * 9 + 0] = -lam; Bn[8 * 9 + 1] = -lam; Bn[8 * 9 + 2] = -lm2; Bn[7 * 9 + 4] = -mu; Bn[6 * 9 + 5] = -mu;
-      Bn[5 * 9 + 6] = -irho; Bn[4 * 9 + 7] = -irho; Bn[2 * 9 + 8] = -irho;
-    }
   }
 
   __device__ static void eigenvalues(const double* Q, int /*d*/, double* lambda) {

@@ -104,8 +104,9 @@ struct CKCfg : Shape<DIM, N, PDE> {
   static constexpr bool kDirRounds = NU == S::b;
   // Blocks per SM of the register budget: three where a block is one cell of
   // N = 5 in 3D (27^3, planes PL apart: 0.753 ms, with two 0.793, four 0.775), else 512 threads
-  // (N=4 with five blocks of 125 threads 208 us, with four 206).
-  static constexpr int BLOCKS = S::P <= 128 ? 4 : PDE::kPointSource ? 2 : 3;  // (the point source's code needs more)
+  // (N=4 with five blocks of 125 threads 208 us, with four 206). The point source's
+  // code needs more: two blocks at 3D N=5, three at 3D N=3 (30^3 324 us, with four, which spill, 337).
+  static constexpr int BLOCKS = S::P <= 128 ? (PDE::kPointSource && DIM == 3 ? 3 : 4) : PDE::kPointSource ? 2 : 3;
   static constexpr int NREG = regs_for_blocks<THREADS, BLOCKS>();
   // the second direction's fluxes lie behind the first's where the planes up to
   // its gradient components hold both (few components or no parameters: in the
@@ -152,60 +153,63 @@ __device__ bool point_source_in_cell(const Geometry& geo, const double* c, const
   return in;
 }
 
-// pointSource (2d/pointSource.cpph:30-127, 3d/pointSource.cpph:28-143) at
-// node p of the cell of centre c and widths h, time slot n (0: t; n >= 1:
-// Gauss-Legendre time node n - 1 of [t, t + dt]): the PDE's source at the
-// node's position, projected onto the node's basis function at the source's
-// reference coordinates and divided by the node's quadrature weight and the
-// cell's widths; zero where the source lies outside the closed cell. The
-// reference's operations in its order, rounded one by one.
+// pointSource (2d/pointSource.cpph:30-127, 3d/pointSource.cpph:28-143) at one
+// node of the cell of centre c and widths h: the PDE's source at the node's
+// position, projected onto the node's basis function at the source's reference
+// coordinates (phi) and divided by the node's quadrature weight and the cell's
+// widths (den); zero where the source lies outside the closed cell. The
+// reference's operations in its order, rounded one by one; phi and den, which
+// do not depend on the time, once per node (a small mesh waits for the cell with
+// the source: 3^3 cells of 3D N=5 75 -> 32 us, 9^2 of 2D N=5 52 -> 20).
 template <int DIM, int N, class PDE>
-__device__ void node_point_source(const Geometry& geo, const double* c, const double* h, int p, double t, double dt,
-                                  int n, double* out) {
-  constexpr int b = N + 1;
-  const OrderTables& T = c_tab[N];
-  const int ix = p % b, iy = (p / b) % b, iz = DIM == 3 ? p / (b * b) : 0;
-  const double tn = n == 0 ? t : __dadd_rn(__dmul_rn(dt, T.x[n - 1]), t);
-  double x[3] = {0.0, 0.0, 0.0}, x0[3];
-  x[0] = __dadd_rn(c[0], __dmul_rn(h[0], __dsub_rn(T.x[ix], 0.5)));
-  x[1] = __dadd_rn(c[1], __dmul_rn(h[1], __dsub_rn(T.x[iy], 0.5)));
-  if (DIM == 3) x[2] = __dadd_rn(c[2], __dmul_rn(h[2], __dsub_rn(T.x[iz], 0.5)));
-  PDE::pointSource(x, tn, dt, out, x0, geo.ps);
-  double xr[3] = {0.0, 0.0, 0.0};
-  bool in = true;
+struct NodePointSource {
+  double x[3], phi, den;
+  bool in;
+  const Geometry& geo;
+  __device__ NodePointSource(const Geometry& g, const double* c, const double* h, int p) : geo(g) {
+    constexpr int b = N + 1;
+    const OrderTables& T = c_tab[N];
+    const int ix = p % b, iy = (p / b) % b, iz = DIM == 3 ? p / (b * b) : 0;
+    x[0] = __dadd_rn(c[0], __dmul_rn(h[0], __dsub_rn(T.x[ix], 0.5)));
+    x[1] = __dadd_rn(c[1], __dmul_rn(h[1], __dsub_rn(T.x[iy], 0.5)));
+    x[2] = DIM == 3 ? __dadd_rn(c[2], __dmul_rn(h[2], __dsub_rn(T.x[iz], 0.5))) : 0.0;
+    double x0[3], xr[3] = {0.0, 0.0, 0.0};
+    PDE::sourcePosition(geo.ps, x0);
+    in = true;
 #pragma unroll
-  for (int e = 0; e < DIM; e++) {
-    xr[e] = __ddiv_rn(__dsub_rn(x0[e], __dsub_rn(c[e], __ddiv_rn(h[e], 2.0))), h[e]);
-    in = in && xr[e] >= 0.0 && xr[e] <= 1.0;
+    for (int e = 0; e < DIM; e++) {
+      xr[e] = __ddiv_rn(__dsub_rn(x0[e], __dsub_rn(c[e], __ddiv_rn(h[e], 2.0))), h[e]);
+      in = in && xr[e] >= 0.0 && xr[e] <= 1.0;
+    }
+    if (DIM == 3) {
+      phi = __dmul_rn(__dmul_rn(lagrange_at<N>(iz, xr[2]), lagrange_at<N>(iy, xr[1])), lagrange_at<N>(ix, xr[0]));
+      den = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(T.w[iz], h[2]), T.w[iy]), h[1]), T.w[ix]), h[0]);
+    } else {
+      phi = __dmul_rn(lagrange_at<N>(iy, xr[1]), lagrange_at<N>(ix, xr[0]));
+      den = __dmul_rn(__dmul_rn(__dmul_rn(T.w[iy], h[1]), T.w[ix]), h[0]);
+    }
   }
-  double phi, den;
-  if (DIM == 3) {
-    phi = __dmul_rn(__dmul_rn(lagrange_at<N>(iz, xr[2]), lagrange_at<N>(iy, xr[1])), lagrange_at<N>(ix, xr[0]));
-    den = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(T.w[iz], h[2]), T.w[iy]), h[1]), T.w[ix]), h[0]);
-  } else {
-    phi = __dmul_rn(lagrange_at<N>(iy, xr[1]), lagrange_at<N>(ix, xr[0]));
-    den = __dmul_rn(__dmul_rn(__dmul_rn(T.w[iy], h[1]), T.w[ix]), h[0]);
+  // at time slot n (0: t; n >= 1: Gauss-Legendre time node n - 1 of [t, t + dt])
+  __device__ void at(double t, double dt, int n, double* out) const {
+    double x0[3];
+    PDE::pointSource(x, n == 0 ? t : __dadd_rn(__dmul_rn(dt, c_tab[N].x[n - 1]), t), dt, out, x0, geo.ps);
+#pragma unroll
+    for (int v = 0; v < PDE::nVar; v++) out[v] = in ? __ddiv_rn(__dmul_rn(phi, out[v]), den) : 0.0;
   }
+  // sum over the time slots n = 1..b of w[n-1] * pointSource (the time integral
+  // the predictor adds, 3d/spaceTimePredictorLinear.cpph:77-90 and :294-308)
+  __device__ void sum(double t, double dt, double* s) const {
 #pragma unroll
-  for (int v = 0; v < PDE::nVar; v++) out[v] = in ? __ddiv_rn(__dmul_rn(phi, out[v]), den) : 0.0;
-}
-
-// sum over the time slots n = 1..b of w[n-1] * pointSource (the time
-// integral the predictor adds, 3d/spaceTimePredictorLinear.cpph:77-90 and
-// :294-308)
-template <int DIM, int N, class PDE>
-__device__ void node_point_source_sum(const Geometry& geo, const double* c, const double* h, int p, double t,
-                                      double dt, double* sum) {
-  const OrderTables& T = c_tab[N];
+    for (int v = 0; v < PDE::nVar; v++) s[v] = 0.0;
+#pragma unroll 1
+    for (int n = 1; n < N + 2; n++) {
+      double val[PDE::nVar];
+      at(t, dt, n, val);
 #pragma unroll
-  for (int v = 0; v < PDE::nVar; v++) sum[v] = 0.0;
-  for (int n = 1; n < N + 2; n++) {
-    double val[PDE::nVar];
-    node_point_source<DIM, N, PDE>(geo, c, h, p, t, dt, n, val);
-#pragma unroll
-    for (int v = 0; v < PDE::nVar; v++) sum[v] = __dadd_rn(sum[v], __dmul_rn(T.w[n - 1], val[v]));
+      for (int v = 0; v < PDE::nVar; v++) s[v] = __dadd_rn(s[v], __dmul_rn(c_tab[N].w[n - 1], val[v]));
+    }
   }
-}
+};
 
 template <int DIM, int N, class PDE, int NREG = CKCfg<DIM, N, PDE>::NREG>
 __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
     // (3d/spaceTimePredictorLinear.cpph:77-90)
     if (here) {
       double psw[nV];
-      node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
+      NodePointSource<DIM, N, PDE>(geo, pc, ph, p).sum(pt, dt, psw);
 #pragma unroll
       for (int v = 0; v < nV; v++) own[PT.at[v]] = qh[v] = __dadd_rn(qh[v], __dmul_rn(dt, psw[v]));
     }
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
 #pragma unroll
     for (int v = 0; v < nV; v++) qn[v] = 0.0;
     if constexpr (PS)  // level 1 starts from the point source's value at t (:93-101)
-      if (here && i == 0) node_point_source<DIM, N, PDE>(geo, pc, ph, p, pt, dt, 0, qn);
+      if (here && i == 0) NodePointSource<DIM, N, PDE>(geo, pc, ph, p).at(pt, dt, 0, qn);
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
       double B[nV];
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(CKCfg<DIM, N, PDE>::THREADS) __maxnreg__(NREG)
   double du[nV];
   double psw[nV];
   if constexpr (PS)
-    if (here) node_point_source_sum<DIM, N, PDE>(geo, pc, ph, p, pt, dt, psw);
+    if (here) NodePointSource<DIM, N, PDE>(geo, pc, ph, p).sum(pt, dt, psw);
 #pragma unroll
   for (int v = 0; v < nV; v++) du[v] = 0.0;
   const double w = (DIM == 3 ? T.w[z] * T.w[y] : T.w[y]) * T.w[x];

@@ -183,6 +183,8 @@ struct KernelSet {
   bool point_source;  // the PDE has a point source (usePointSource)
   bool tmem;          // variants 0 and 8 are the tensor-memory form, which counts its sweeps itself
   int predictor_launches(int variant) const { return linear || (tmem && (variant == 0 || variant == 8)) ? 1 : 2; }
+  // the variant whose launch `variant` repeats (itself: a kernel of its own)
+  int same_as(int variant) const { return (linear && variant == 1) || (tmem && variant == 8) ? 0 : variant; }
 };
 
 template <int DIM, int N, class PDE>
@@ -945,8 +947,12 @@ int exa_solver_autotune(exa_solver* s, int ncells, double* variant_ms, int* chos
   int best = 0;
   double best_ms = 1e300;
   for (int v = 0; v < kAllVariants && rc == EXA_OK; v++) {
-    if (variant_is_mixed(v) || (k.linear && v > 1)) {  // mixed: changes the results; linear: two shapes
+    if (variant_is_mixed(v) || (k.linear && v > 1)) {  // mixed: changes the results; linear: 0 and 1 only
       if (variant_ms) variant_ms[v] = -1.0;
+      continue;
+    }
+    if (const int same = k.same_as(v); same != v) {  // the same kernel is not timed twice
+      if (variant_ms) variant_ms[v] = variant_ms[same];
       continue;
     }
     float ms = 0.f, tot = 0.f;

@@ -88,7 +88,9 @@ int exa_solver_sizes(const exa_solver* s, int* sizes4);
 /* Variant 8 keeps the Picard iterate in the SM's tensor memory (PDEs of five
  * state variables without parameters and source terms; other shapes run
  * variant 6 under this number). Variant 0, what a solver starts with, is the
- * same form where variant 8 has it, the node form elsewhere. */
+ * same form where variant 8 has it, the node form elsewhere. The linear
+ * predictor has one shape, under 0 and 1. Two variants that are one kernel are
+ * timed once: both get its figure and the lower number is the one chosen. */
 /* Variants beyond the autotuned ones (exa_solver_set_variant only): the
  * mixed-precision predictor. Its first Picard sweep is the FP64 sweep; every
  * later sweep forms the flux increment F(q^k) - F(q^(k-1)) in FP64 and runs

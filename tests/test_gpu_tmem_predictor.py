@@ -61,3 +61,12 @@ def test_mixed_sweep_counts_vs_oracle(eb, dim, order, n, variant):
         assert np.max(np.abs(qb[c] - o["lQhbnd"])) <= 1e-12 * np.max(np.abs(o["lQhbnd"]))
         assert np.max(np.abs(fb[c] - o["lFhbnd"])) <= 1e-12 * np.max(np.abs(o["lFhbnd"]))
         assert np.max(np.abs(du[c] - o["lduh"])) <= 1e-12 * max(np.max(np.abs(o["lduh"])), scale)
+
+
+@pytest.mark.parametrize("pde,twin", [(0, 8), (2, 1)])
+def test_autotune_times_one_kernel_once(eb, pde, twin):
+    """variants 0 and 8 of the Euler predictor are one kernel, 0 and 1 of the linear one"""
+    for _ in range(3):
+        s = eb.Solver(2, 3, pde)
+        chosen, ms = s.autotune(64)
+        assert ms[twin] == ms[0] > 0 and chosen != twin and s.variant == chosen

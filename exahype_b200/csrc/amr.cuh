@@ -39,6 +39,8 @@ namespace exa {
 // [n][i]. A block reads one matrix with block-uniform addresses, so the
 // coefficients come from the constant cache by broadcast.
 constexpr bool amr_has(int N) { return N == 3 || N == 4 || N == 5 || N == 7; }
+// (an order added to the solvers is added here, to LineTablesAll and
+// ProjTablesAll, and to upload_tables)
 constexpr int amr_off(int N) { return N <= 3 ? 0 : amr_off(N - 1) + (amr_has(N - 1) ? N * N : 0); }
 constexpr int kAmrSq = amr_off(8);  // sum of (N+1)^2 over the orders
 __constant__ double c_amr_fine[3 * kAmrSq];
@@ -62,6 +64,7 @@ __constant__ double c_amr_equi[kAmrSq];
 // per row, free of bank conflicts too (half-warps, 64-bit accesses).
 template <int b, int NAX, int NV>
 struct TensorCfg {
+  static_assert(amr_has(b - 1), "no transfer tables of this order");
   static constexpr int LINES = NV * ipow(b, NAX - 1), SIZE = LINES * b;
   static constexpr int ROUNDS = b >= 8 ? (LINES + 319) / 320 : (LINES + 255) / 256;
   static constexpr int THREADS = ((LINES + ROUNDS - 1) / ROUNDS + 31) / 32 * 32;

@@ -126,6 +126,7 @@ struct ProjTablesAll {
 __constant__ ProjTablesAll c_proj;
 template <int N>
 __device__ __forceinline__ const ProjTables<N>& proj_tab() {
+  static_assert(N == 3 || N == 4 || N == 5 || N == 7, "no projection tables of this order");
   if constexpr (N == 3) return c_proj.n3;
   else if constexpr (N == 4) return c_proj.n4;
   else if constexpr (N == 5) return c_proj.n5;

@@ -38,6 +38,7 @@ struct LineTablesAll {
 __constant__ LineTablesAll c_line;
 template <int N>
 __device__ __forceinline__ const LineTables<N>& line_tab() {
+  static_assert(N == 3 || N == 4 || N == 5 || N == 7, "no line tables of this order");
   if constexpr (N == 3) return c_line.n3;
   else if constexpr (N == 4) return c_line.n4;
   else if constexpr (N == 5) return c_line.n5;

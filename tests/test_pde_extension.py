@@ -1,7 +1,8 @@
 """PDE structs of other shapes than the library's own compile against the kernels
 (CPU) and give right results (GPU): a linear PDE without parameters, one with
 unequal numbers of gradient components per direction, and one with more than 16
-values per node in the Riemann solver.
+values per node in the Riemann solver. An order without transfer tables does not
+compile (it would read another order's).
 
 Bounds: the same sums in another order, 1e-12 of the largest value (the derivative
 tables are read from the same generator)."""
@@ -29,6 +30,19 @@ def compile_ext(out, *flags):
 @pytest.mark.skipif(not NVCC, reason="needs nvcc")
 def test_other_pde_shapes_compile(tmp_path):
     compile_ext(tmp_path / "ext.o", "-c")
+
+
+@pytest.mark.skipif(not NVCC, reason="needs nvcc")
+def test_orders_without_tables_do_not_compile(tmp_path):
+    src = tmp_path / "t.cu"
+    src.write_text('#include "amr.cuh"\n'
+                   "template __global__ void exa::plot_vertex_kernel<2, ORDER, 5>(const double*, double*, int);\n")
+    run = lambda order: subprocess.run(  # noqa: E731
+        [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC,
+         "-DORDER=%d" % order, "-c", str(src), "-o", str(tmp_path / "t.o")], capture_output=True, text=True)
+    assert run(5).returncode == 0
+    r = run(6)
+    assert r.returncode != 0 and "no transfer tables" in r.stderr
 
 
 @pytest.fixture(scope="module")

@@ -95,6 +95,9 @@ struct TmemCfg : Shape<DIM, N, PDE> {
                                 MINB * (SMEM + 2048) <= 228 * 1024;
   static_assert(S::P * S::nV <= SFJ, "the time-averaged state is staged in the second slice buffer");
   static_assert(kByDir || sstride(0) == sstride(DIM - 1), "items over all directions: one stride");
+  // items over all directions go by p + r P: a thread past the last node would take
+  // another's item and contract its line a second time, in place
+  static_assert(kByDir || THREADS == CPB * S::P, "items over all directions: a node for every thread");
 };
 
 template <int DIM, int N, class PDE, bool FEW>

@@ -45,6 +45,20 @@ def test_orders_without_tables_do_not_compile(tmp_path):
     assert r.returncode != 0 and "no transfer tables" in r.stderr
 
 
+@pytest.mark.skipif(not NVCC, reason="needs nvcc")
+def test_tensor_memory_predictor_refuses_idle_threads(tmp_path):
+    """order 2 in 2D: 126 nodes in a block of 128 threads and more lines than nodes"""
+    src = tmp_path / "t.cu"
+    src.write_text('#include "aderdg.cuh"\n#include "predictor_tmem.cuh"\n'
+                   "static_assert(exa::TmemCfg<2, ORDER, exa::EulerPDE>::THREADS == 128);\n")
+    run = lambda order: subprocess.run(  # noqa: E731
+        [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC,
+         "-DORDER=%d" % order, "-c", str(src), "-o", str(tmp_path / "t.o")], capture_output=True, text=True)
+    assert run(3).returncode == 0
+    r = run(2)
+    assert r.returncode != 0 and "a node for every thread" in r.stderr
+
+
 @pytest.fixture(scope="module")
 def ext(tmp_path_factory):
     torch = pytest.importorskip("torch")

@@ -355,8 +355,10 @@ struct Launch {
       rc = launch_lines<false, 2, false, kSlices2 ? 2 : 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
     else if (variant == 6 || variant == 7 || variant == 8)
       rc = launch_lines<false, 1, false, kSlices1 ? 2 : 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
-    else
+    else if constexpr (!kTmem)
       rc = launch_pred<false, 1, 1>(luh, qb, fb, du, iters, dt, g, n, list, cnt, tmp, st);
+    else  // (0 went to the tensor-memory form above)
+      rc = fail(EXA_ERR_ARG, "predictor: no variant " + std::to_string(variant));
     if (rc) return rc;
     if (acc && iters) {
       sweep_count_kernel<DIM, N, PDE><<<std::min(1024, (n + 255) / 256), 256, 0, st>>>(iters, list, n, cnt, acc);

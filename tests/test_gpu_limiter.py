@@ -118,9 +118,10 @@ def test_limiting_mesh_2d_outflow(eb, dim, order, cells, steps, helper, cure):
     (2, 4, (14, 14), 30, 1, 2),
 ])
 def test_limiting_mesh_2d_tensor_memory_predictor(eb, dim, order, cells, steps, helper, cure):
-    """the same comparison with the line-form predictor that keeps the Picard
-    iterate in tensor memory (variant 8), run on the limiting mesh's
-    device-compacted cell lists with several cells per block"""
+    """the same comparison with the predictor that keeps the Picard iterate in
+    tensor memory (variant 8), run on the limiting mesh's device-compacted cell
+    lists: one cell per block (two at order 3) on meshes of at most 296 cells,
+    several on the larger one"""
     _, g, o = make_pair(eb, dim, order, cells, 0, helper, cure, seed=3, variant=8)
     compare(g, o, dim, order, "init")
     for k in range(steps):
@@ -129,11 +130,11 @@ def test_limiting_mesh_2d_tensor_memory_predictor(eb, dim, order, cells, steps, 
         compare(g, o, dim, order, "step %d" % (k + 1), check_lim=(k % 5 == 4))
 
 
-@pytest.mark.parametrize("order,cells,steps,variant", [(3, (6, 6, 6), 10, None), (5, (5, 5, 5), 6, None),
+@pytest.mark.parametrize("order,cells,steps,variant", [(3, (6, 6, 6), 10, 3), (5, (5, 5, 5), 6, 3),
                                                      (3, (6, 6, 6), 10, 8), (5, (5, 5, 5), 6, 8)])
 def test_limiting_mesh_3d_outflow(eb, order, cells, steps, variant):
-    """variant 8: the tensor-memory predictor on the limiting mesh's cell lists
-    (3D N=5: one cell per block; N=3: four)"""
+    """variant 3: the node form; 8: the tensor-memory predictor on the limiting
+    mesh's cell lists (one cell per block, as for any mesh of at most 296 cells)"""
     _, g, o = make_pair(eb, 3, order, cells, 0, 1, 0, seed=1, variant=variant)
     compare(g, o, 3, order, "init")
     for k in range(steps):

@@ -97,8 +97,8 @@ def test_musclhancock_update_vs_oracle(eb, dim, order, n):
 
 
 def test_musclhancock_scratch_limits(eb):
-    """3D needs scratch: less than one block's share is refused on the host;
-    room for a single block gives the same result as the full grid"""
+    """3D asks for scratch: less than one block's share is refused on the host; one
+    share is enough for any list (the kernel keeps its working set on chip)"""
     rng = np.random.default_rng(5)
     dim, order, n = 3, 3, 9
     E = 2 * order + 5
@@ -110,7 +110,7 @@ def test_musclhancock_scratch_limits(eb):
     outs = []
     for nbytes in (full, None):
         g_lim, g_old = dev(lim), dev(np.zeros_like(lim))
-        if nbytes is None:  # room for exactly one block: the grid-stride loop does all cells
+        if nbytes is None:  # one share
             one = s.fv_musclhancock_scratch_bytes(1)
             scratch = torch.empty(one // 8, dtype=torch.float64, device="cuda")
             s.fv_musclhancock_update(g_lim, g_old, None, g_dt, dx, n, None, scratch, one)

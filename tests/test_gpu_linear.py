@@ -59,7 +59,7 @@ def elastic_state(golden, var, par, n):
     return np.concatenate([golden[g + var].reshape(n, 9), golden[g + par].reshape(n, 3)], axis=1)
 
 
-@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("variant", [0, 1])  # one kernel under two numbers
 def test_predictor_linear_golden_gpu(eb, golden, variant):
     """ElasticityKernelTest2D::testSpaceTimePredictorLinear (N = 4) replayed on
     the GPU: time averages and boundary extrapolations"""
@@ -99,14 +99,12 @@ def test_riemann_and_volume_linear_golden_gpu(eb, golden):
     np.testing.assert_allclose(host(du), golden[g + "testVolumeIntegralLinear/lduh_OUT"], rtol=0, atol=1e-9)
 
 
-@pytest.mark.parametrize("variant", [0, 1])
 @pytest.mark.parametrize("dim,N", [(2, 3), (2, 4), (2, 5), (3, 3), (3, 4), (3, 5)])
-def test_linear_kernels_vs_oracle(eb, dim, N, variant):
+def test_linear_kernels_vs_oracle(eb, dim, N):
     """predictor + volume integral, Riemann solver and corrector (linear
     surface integral, update, admissible step) on random elastic cells"""
     rng = np.random.default_rng(100 * dim + N)
     s = eb.Solver(dim, N, eb.PDE_ELASTIC)
-    s.variant = variant
     o = pyoracle.Kernels(dim, N, pde=2)
     b = N + 1
     P, F, n = b ** dim, b ** (dim - 1), 37

@@ -1,10 +1,14 @@
 """The plane-by-plane 3D MUSCL-Hancock update at the orders the limiter-kernel
-tests do not reach (4 and 7: other plane sizes, other remainders of the block)
-and for one cell and more cells than the device holds blocks, with the check
-and the bound of test_gpu_limiter_kernels (1e-12 relative max-norm)."""
+tests do not reach (4 and 7: other plane sizes, other remainders of the block),
+with the check and the bound of test_gpu_limiter_kernels (1e-12 relative
+max-norm); for lists of any length, which the kernel-level call gives a block per
+cell; and on limiting meshes with more FV-active cells than the device holds
+blocks, where a block takes several."""
 import numpy as np
 import pytest
 
+import pyoracle
+import test_gpu_limiter as lim
 import test_gpu_limiter_kernels as lk
 from test_gpu_limiter_kernels import eb  # noqa: F401  (fixture)
 
@@ -36,3 +40,27 @@ def test_many_cells_equal_single_calls(eb):  # noqa: F811
         one, prev = lk.dev(lim[c:c + 1]), lk.dev(np.zeros_like(lim[:1]))
         s.fv_musclhancock_update(one, prev, None, dt, dx, 1, None, scratch, scratch.numel() * 8)
         assert np.array_equal(lk.host(one)[0], lk.host(got)[c])
+
+
+def test_blocks_take_several_cells(eb):  # noqa: F811
+    """3D order 7 (one block an SM): a rough state under a maximum principle without
+    slack makes every cell FV-active, so that blocks walk their patches one after
+    the other; first in the recomputation, then in the update"""
+    order, cells = 7, (6, 6, 6)
+    rng = np.random.default_rng(11)
+    n = int(np.prod(cells))
+    luh = np.zeros((n, 8 ** 3, 5))
+    luh[..., 0] = 1.0 + 0.01 * rng.random(luh.shape[:2])
+    luh[..., 1:4] = 0.01 * (rng.random(luh.shape[:2] + (3,)) - 0.5)
+    luh[..., 4] = 2.5 + 0.01 * rng.random(luh.shape[:2])
+    g = eb.LimitingMesh(eb.Solver(3, order), cells, [0.0] * 3, [1.0] * 3, 0, relax=0.0, scale=0.0)
+    o = pyoracle.LimitingMesh(3, order, cells, [1.0] * 3, 0, relax=0.0, scale=0.0, nthreads=8)
+    for m in (g, o):
+        m.set_solution(luh)
+        m.init(0.0)
+    for k in range(2):
+        g.step(1)
+        o.step(1)
+        status = lim.compare(g, o, 3, order, "step %d" % (k + 1))
+        assert np.sum(status >= 2) > torch.cuda.get_device_properties(0).multi_processor_count
+    assert o.state()["irregular_steps"] >= 1

@@ -63,12 +63,10 @@ def solver(eb, dim, N, ps=PS):
     return s
 
 
-@pytest.mark.parametrize("variant", [0, 1])
 @pytest.mark.parametrize("dim,N", [(2, 3), (2, 5), (3, 3), (3, 5)])
-def test_predictor_vs_oracle_and_reference(eb, dim, N, variant):
+def test_predictor_vs_oracle_and_reference(eb, dim, N):
     rng = np.random.default_rng(dim * 13 + N)
     s = solver(eb, dim, N)
-    s.variant = variant
     b = N + 1
     P, F = b ** dim, b ** (dim - 1)
     dx = [0.1, 0.12, 0.09][:dim]

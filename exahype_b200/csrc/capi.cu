@@ -2699,17 +2699,19 @@ int exa_fv_musclhancock_update_noalloc(const exa_solver* s, double* lim, double*
                    (cudaStream_t)stream);
 }
 
-// side streams of the mesh stream's priority, and the events that fork and join them
+// side streams of the mesh stream's priority, and the events that fork and join
+// them; where a new one cannot be had, those that are there stay
 static cudaError_t lmesh_side_streams(exa_lmesh* lm) {
   int prio = 0;
+  cudaStream_t side[2] = {nullptr, nullptr};
   cudaError_t e = cudaStreamGetPriority(lm->m->stream, &prio);
-  for (cudaStream_t& x : lm->side) {
-    if (x) cudaStreamDestroy(x);
-    x = nullptr;
+  for (cudaStream_t& x : side)
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio);
-  }
   for (cudaEvent_t* ev : {&lm->fork, &lm->ready, &lm->joined[0], &lm->joined[1]})
     if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) std::swap(side, lm->side);
+  for (cudaStream_t x : side)
+    if (x) cudaStreamDestroy(x);
   return e;
 }
 

@@ -38,3 +38,22 @@ def test_statuses_vs_oracle(eb, dim, cells, bc, layers, steps):
         o.step(1)
         assert np.array_equal(g.status(), o.status())
     assert np.linalg.norm(g.get_solution() - o.get_solution()) <= 1e-11 * np.linalg.norm(o.get_solution())
+
+
+def test_priority_between_steps(eb):
+    """a new stream, and new side streams, between steps change no result"""
+    from exahype_b200 import problems
+    u, fv, _ = problems.explosion(2, 3, (12, 11), seed=4)
+    out = []
+    for levels in ((), (1, 3, 0)):
+        m = eb.LimitingMesh(eb.Solver(2, 3), (12, 11), (0.0, 0.0), (1.0, 1.0), 0)
+        m.set_solution(u)
+        m.set_fv_initial(fv)
+        m.init(0.0)
+        for k in range(3):
+            m.step(1)
+            if levels:
+                m.set_priority(levels[k])
+            m.run_until(1.0, 2)
+        out.append((m.get_solution(), m.status(), m.state()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]

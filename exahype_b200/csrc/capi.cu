@@ -2503,7 +2503,17 @@ struct LimLaunch {
 
   // One limiting step. run (optional, device): when it holds 0 every launch
   // of the step returns at once (run_until replays captured steps past t_end).
+  // A step that fails on the way joins what it forked too: the mesh stream alone
+  // orders what comes after it, the release of the mesh's memory included.
   static int step_launch(exa_lmesh* lm, int* run) {
+    const int rc = step_forked(lm, run);
+    if (rc)
+      for (int i : {0, 1})
+        if (cudaEventRecord(lm->joined[i], lm->side[i]) == cudaSuccess)
+          cudaStreamWaitEvent(lm->m->stream, lm->joined[i], 0);
+    return rc;
+  }
+  static int step_forked(exa_lmesh* lm, int* run) {
     exa_mesh* m = lm->m;
     const KernelSet& k = m->s->k;
     const int n = m->ncells;

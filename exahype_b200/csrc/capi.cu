@@ -2316,9 +2316,9 @@ struct LimLaunch {
   using PDE = EulerPDE;
   using L = LimShape<DIM, N>;
   using MC = typename std::conditional<DIM == 2, MusclCfg<N>, Muscl3Cfg<N>>::type;
-  // The scratch that the kernel-level update asks for per block in 3D: the
-  // evolved states and edge fluxes of a whole patch. The kernel keeps them on
-  // chip; the size stays the interface's, and a call with less is refused.
+  // The scratch that the kernel-level update asks for in 3D, whatever the number
+  // of cells: the evolved states and edge fluxes of one patch. The kernel keeps
+  // them on chip; the size stays the interface's, and a call with less is refused.
   static constexpr size_t kShare =
       DIM == 2 ? 0 : (size_t)ipow(L::B + 2, 3) * 6 * L::nV + (size_t)3 * (L::B + 1) * L::B * L::B * L::nV;
   static const void* muscl_fn() {
@@ -2382,23 +2382,13 @@ struct LimLaunch {
     if constexpr (kShare > 0)
       if (needs_scratch && (!scratch || scratch_doubles_avail < kShare))
         return fail(EXA_ERR_ARG, "exa_fv_musclhancock_update: scratch holds " +
-                                     std::to_string(scratch_doubles_avail * 8) + " bytes, one block needs " +
+                                     std::to_string(scratch_doubles_avail * 8) + " bytes, the call asks for " +
                                      std::to_string(kShare * 8));
     muscl_launch(n, st, list, nullptr, n, lim, lim_old, luh, g, dt, nullptr);
     EXA_LAUNCHED();
     return EXA_OK;
   }
-  static int scratch_bytes_for(int n, size_t* bytes) {
-    if (kShare == 0 || n <= 0) {
-      *bytes = 0;
-      return EXA_OK;
-    }
-    int grid = 0;
-    int rc = muscl_grid(n, &grid);
-    if (rc) return rc;
-    *bytes = (size_t)grid * kShare * sizeof(double);
-    return EXA_OK;
-  }
+  static size_t scratch_bytes_for(int n) { return n > 0 ? kShare * sizeof(double) : 0; }
   static int project_call(double* luh, double* lim, int n, const int* list, int to_fv, cudaStream_t st) {
     if (n <= 0) return EXA_OK;
     int rc = attrs();
@@ -2627,7 +2617,7 @@ struct LimOps {
   size_t LS, PB;
   int (*muscl)(double*, double*, double*, const double*, Geometry, int, const int*, const double*, size_t, bool,
                cudaStream_t);
-  int (*scratch_bytes)(int, size_t*);
+  size_t (*scratch_bytes)(int);
   int (*project)(double*, double*, int, const int*, int, cudaStream_t);
 };
 
@@ -2680,7 +2670,8 @@ int exa_fv_musclhancock_scratch_bytes(const exa_solver* s, int ncells, size_t* b
   int rc = lim_ops_of(s, "exa_fv_musclhancock_scratch_bytes", &ops);
   if (rc) return rc;
   if (!bytes || ncells < 0) return fail(EXA_ERR_ARG, "exa_fv_musclhancock_scratch_bytes: bad argument");
-  return ops.scratch_bytes(ncells, bytes);
+  *bytes = ops.scratch_bytes(ncells);
+  return EXA_OK;
 }
 
 int exa_fv_musclhancock_update(const exa_solver* s, double* lim, double* lim_old, double* luh, const double* dt_dev,

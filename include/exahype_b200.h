@@ -368,10 +368,10 @@ int exa_project_on_dg_space(const exa_solver* s, const double* lim, double* luh,
  * listed cell lim_old <- lim (ghost layers included; the caller has filled
  * them), then lim <- the MUSCL-Hancock update of lim_old by *dt_dev, and, when
  * luh is not NULL, luh <- projectOnDGSpace(lim). For 3D patches the caller
- * passes device scratch of exa_fv_musclhancock_scratch_bytes(s, ncells) bytes
- * (less than one block's share is an error; the present kernels keep their
- * working set on chip and do not touch it); 2D needs none (scratch may be
- * NULL). */
+ * passes device scratch of exa_fv_musclhancock_scratch_bytes(s, ncells) bytes,
+ * one patch's work arrays for any ncells > 0 (less is an error; the present
+ * kernels keep their working set on chip and do not touch it); 2D needs none
+ * (scratch may be NULL). */
 int exa_fv_musclhancock_scratch_bytes(const exa_solver* s, int ncells, size_t* bytes);
 int exa_fv_musclhancock_update(const exa_solver* s, double* lim, double* lim_old, double* luh, const double* dt_dev,
                                const double* dx, int ncells, const int* cell_list, void* scratch, size_t scratch_bytes,

@@ -97,8 +97,8 @@ def test_musclhancock_update_vs_oracle(eb, dim, order, n):
 
 
 def test_musclhancock_scratch_limits(eb):
-    """3D asks for scratch: less than one block's share is refused on the host; one
-    share is enough for any list (the kernel keeps its working set on chip)"""
+    """3D asks for scratch: one patch's share whatever the number of cells; less is
+    refused on the host, more is taken"""
     rng = np.random.default_rng(5)
     dim, order, n = 3, 3, 9
     E = 2 * order + 5
@@ -106,17 +106,13 @@ def test_musclhancock_scratch_limits(eb):
     s = eb.Solver(dim, order)
     g_dt = dev(np.array([1e-4]))
     dx = [0.05, 0.05, 0.05]
-    full = s.fv_musclhancock_scratch_bytes(n)
+    share = s.fv_musclhancock_scratch_bytes(1)
+    assert share > 0 and s.fv_musclhancock_scratch_bytes(5000) == share and s.fv_musclhancock_scratch_bytes(0) == 0
     outs = []
-    for nbytes in (full, None):
+    for nbytes in (share, n * share):
         g_lim, g_old = dev(lim), dev(np.zeros_like(lim))
-        if nbytes is None:  # one share
-            one = s.fv_musclhancock_scratch_bytes(1)
-            scratch = torch.empty(one // 8, dtype=torch.float64, device="cuda")
-            s.fv_musclhancock_update(g_lim, g_old, None, g_dt, dx, n, None, scratch, one)
-        else:
-            scratch = torch.empty(nbytes // 8, dtype=torch.float64, device="cuda")
-            s.fv_musclhancock_update(g_lim, g_old, None, g_dt, dx, n, None, scratch, nbytes)
+        scratch = torch.empty(nbytes // 8, dtype=torch.float64, device="cuda")
+        s.fv_musclhancock_update(g_lim, g_old, None, g_dt, dx, n, None, scratch, nbytes)
         outs.append(host(g_lim))
     assert np.array_equal(outs[0], outs[1])
     with pytest.raises(eb.ExaError, match="scratch"):

@@ -49,13 +49,14 @@ __constant__ double c_amr_equi[kAmrSq];
 
 // A block works on one tensor of NAX axes with b nodes each and NV values per
 // node: one thread per line of the axis in turn, in ROUNDS rounds where that is
-// more than 256 threads (order 7: 320). The 320 lines of 3D order 7 take one
-// round, the 432 of the elastic state at order 5 two, unrolled (but for sums into
-// global memory): in a loop over the rounds the compiler holds matrix entries in
-// registers across them and spills (transfers of order 7: 96 registers and up
-// to 884 bytes, now 50 and none; 5,832 of them: prolongation 77 -> 54 us,
-// restriction 76 -> 56, vertex projection 71 -> 68). The lines of an axis are
-// disjoint, so every pass works in place in one shared buffer; the first pass
+// more than 256 threads (order 7: 320). In a loop over rounds the compiler holds
+// matrix entries of the transfers in registers across them and spills. So the 320
+// lines of 3D order 7 take one round (96 registers and up to 884 bytes before, now
+// 50 and none; 5,832 transfers: prolongation 77 -> 54 us, restriction 76 -> 56,
+// vertex projection 71 -> 68), and the two rounds of the elastic state at order 5
+// (432 lines) are unrolled, but for sums into global memory and in the vertex
+// projection (20,000 cells 128 us in a loop, 160 unrolled). The lines of an axis
+// are disjoint, so every pass works in place in one shared buffer; the first pass
 // reads its lines from global memory and the last one writes its results there.
 // Consecutive threads take consecutive values of the x rows, so the last
 // axis (of two or three) is written coalesced; the first (x) pass reads each row
@@ -89,10 +90,10 @@ enum class Place { kBuffer, kGlobal, kGlobalAdd };
 // out[.., m, ..] = sum_n M[m][n] in[.., n, ..] along axis AX, M given as a
 // constant-memory pointer and row / column strides (compile-time indices: the
 // coefficients are constant-bank operands). `tid` of `THREADS` threads.
-template <class C, int b, int AX, int RS, int CS, Place FROM, Place TO>
+template <class C, int b, int AX, int RS, int CS, Place FROM, Place TO, bool UNROLL = false>
 __device__ __forceinline__ void apply_axis(const double* src, double* dst, double* buf, const double* M, int tid) {
   constexpr int ROW = C::ROW;
-#pragma unroll(TO == Place::kGlobalAdd ? 1 : C::ROUNDS)
+#pragma unroll(UNROLL && TO != Place::kGlobalAdd ? C::ROUNDS : 1)
   for (int r = 0; r < C::ROUNDS; r++) {
     const int it = tid + r * C::THREADS;
     if (it >= C::LINES) break;
@@ -126,11 +127,11 @@ __device__ __forceinline__ void transfer_axis(const double* src, double* dst, do
   constexpr int b = N + 1, base = 3 * amr_off(N), RS = R ? b : 1, CS = R ? 1 : b;
   const double* tab = R ? c_amr_restr : c_amr_fine;
   if (digit == 0) {
-    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base, tid);
+    apply_axis<C, b, AX, RS, CS, FROM, TO, true>(src, dst, buf, tab + base, tid);
   } else if (digit == 1) {
-    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base + b * b, tid);
+    apply_axis<C, b, AX, RS, CS, FROM, TO, true>(src, dst, buf, tab + base + b * b, tid);
   } else {
-    apply_axis<C, b, AX, RS, CS, FROM, TO>(src, dst, buf, tab + base + 2 * b * b, tid);
+    apply_axis<C, b, AX, RS, CS, FROM, TO, true>(src, dst, buf, tab + base + 2 * b * b, tid);
   }
 }
 

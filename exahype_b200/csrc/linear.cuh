@@ -61,8 +61,8 @@ struct GradPairs {
 // position modulo the 16 banks of 64 bits is chosen by what is read and written
 // together. The residues come from a search over a count of the wavefronts of
 // the three directions' loads (state) and stores (components) with the item
-// orders of the kernel; 966 a level against 1188 with all planes PL apart
-// (882 if nothing met). The shared-memory pipe bounds the kernel (96 % busy
+// orders of the kernel (gen_planes.py); 966 a level against 1188 with all planes
+// PL apart (882 if nothing met). The shared-memory pipe bounds the kernel (96 % busy
 // before): 27^3 N=5 757 -> 720 us.
 template <int PLANES, int PL, int CELL, bool PLACED>
 struct CKPlanes {

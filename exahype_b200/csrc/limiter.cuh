@@ -798,7 +798,10 @@ struct PostCfg {
   static constexpr bool kWarp = DIM == 2;
   using Group = typename std::conditional<kWarp, WarpGroup, BlockGroup>::type;
   static constexpr int CELLS = kWarp ? THREADS / 32 : 1;
-  static constexpr int BLOCKS = !kWarp ? 1 : N == 7 ? 5 : 8;  // per SM, of the post-update kernel's registers
+  // per SM, of the post-update kernel's registers. 3D states none: 128 to 135
+  // registers a thread, lines instead of an output per thread (a limiting step of
+  // 12^3 N=3 with its other kernels 503 -> 271 us, 9^3 N=5 864 -> 337, 7^3 N=7 2031 -> 539)
+  static constexpr int BLOCKS = !kWarp ? 1 : N == 7 ? 5 : 8;
   // per cell: tensor-map scratch, reduction slots (a whole block's), the
   // staged DG solution
   static constexpr int RED = kWarp ? 0 : 2 * THREADS + 10;
@@ -809,8 +812,9 @@ struct PostCfg {
 // Min/max of the observables (the conserved variables) over the
 // Gauss-Legendre nodes, the Gauss-Lobatto nodes and the subcell centres of one
 // cell (findCellLocalMinAndMax + compareWithADERDGSolutionAtGaussLobattoNodes +
-// compareWithADERDGSolutionAtFVSubcellCenters, Limiter.cpp:210-368). Block-wide;
-// every thread ends with the cell's values in mn/mx.
+// compareWithADERDGSolutionAtFVSubcellCenters, Limiter.cpp:210-368). By the whole
+// group; a thread below line_threads ends with the part it saw of variable
+// tid % 5, for block_minmax_lines or warp_minmax_lines to put together.
 template <int DIM, int N, class G = BlockGroup>
 __device__ MinMax local_minmax_lines(const double* u, double* tmp) {
   using L = LimShape<DIM, N>;

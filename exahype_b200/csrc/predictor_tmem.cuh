@@ -28,7 +28,7 @@
 //
 // Bound: latency of the FP64 chains and the barriers between the phases at 14
 // warps per SM (two blocks by registers; the accumulators alone are 60 at
-// N = 5), next the shared-memory pipe (58 %) and the FP64 pipe (38 %). Measured
+// N = 5), next the shared-memory pipe (69 %) and the FP64 pipe (45 %). Measured
 // without gain: overlapping the phases of consecutive pairs in two buffers
 // (fewer barriers, the same chains: 0.96 ms against 0.88 on 27^3 N=5), two
 // threads per node with half of the slices each (twice the warps at 72
